@@ -1,5 +1,5 @@
-// Mamba2 selective state-space scan (SSD recurrence) and the depthwise causal conv + SiLU in front
-// of it, forward and backward, for sm_100a.
+// Mamba2 selective state-space scan (SSD recurrence), forward and backward, for sm_100a (the depthwise conv in
+// front of it is in conv1d.cu).
 //
 //   h_t[p,n] = exp(a_t) * h_{t-1}[p,n] + x_t[p] * b_t[n]        (one state matrix [P, N] per batch x head)
 //   y_t[p]   = sum_n h_t[p,n] * c_t[n]
@@ -199,91 +199,6 @@ __global__ void __launch_bounds__(256) ssd_bwd_kernel(const ScanParams p) {
   }
 }
 
-// ---- depthwise causal conv (K taps) + SiLU ------------------------------------------------------------
-//   u[t, ch] = bias[ch] + sum_k w[ch, k] * x[t - (K-1) + k, ch];   y = u * sigmoid(u)
-template <int K>
-__global__ void conv_fwd_kernel(const float* x, const float* w, const float* bias, float* y, int B, int L, int C) {
-  const long long total = static_cast<long long>(B) * L * C;
-  for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
-       i += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const int ch = static_cast<int>(i % C);
-    const int t = static_cast<int>((i / C) % L);
-    float u = bias != nullptr ? bias[ch] : 0.f;
-#pragma unroll
-    for (int k = 0; k < K; ++k) {
-      const int tt = t - (K - 1) + k;
-      if (tt >= 0) u = fmaf(w[ch * K + k], x[i + static_cast<long long>(tt - t) * C], u);
-    }
-    y[i] = u / (1.f + __expf(-u));
-  }
-}
-
-// dx[t] = sum_k w[k] * du[t + (K-1) - k];  dw / dbias are reduced per channel by a second kernel.
-template <int K>
-__global__ void conv_bwd_dx_kernel(const float* x, const float* w, const float* bias, const float* dy, float* dx,
-                                   float* du_out, int B, int L, int C) {
-  const long long total = static_cast<long long>(B) * L * C;
-  for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
-       i += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const int ch = static_cast<int>(i % C);
-    const int t = static_cast<int>((i / C) % L);
-    float acc = 0.f;
-#pragma unroll
-    for (int k = 0; k < K; ++k) {
-      const int to = t + (K - 1) - k;      // output position that read x[t] through tap k
-      if (to >= L) continue;
-      // recompute u[to] and the SiLU derivative
-      float u = bias != nullptr ? bias[ch] : 0.f;
-#pragma unroll
-      for (int j = 0; j < K; ++j) {
-        const int tt = to - (K - 1) + j;
-        if (tt >= 0) u = fmaf(w[ch * K + j], x[i + static_cast<long long>(tt - t) * C], u);
-      }
-      const float sg = 1.f / (1.f + __expf(-u));
-      const float du = dy[i + static_cast<long long>(to - t) * C] * sg * (1.f + u * (1.f - sg));
-      if (k == K - 1) du_out[i] = du;      // to == t: this thread owns du[t]
-      acc = fmaf(w[ch * K + k], du, acc);
-    }
-    dx[i] = acc;
-  }
-}
-
-// dw[ch, k] = sum_{b,t} du[b,t,ch] * x[b, t-(K-1)+k, ch];  dbias[ch] = sum du.  One block per 32 channels.
-template <int K>
-__global__ void __launch_bounds__(256) conv_bwd_dw_kernel(const float* x, const float* du, float* dw, float* dbias,
-                                                          int B, int L, int C) {
-  __shared__ float part[8][32][K + 1];
-  const int lane = threadIdx.x & 31, wy = threadIdx.x >> 5;
-  const int ch = blockIdx.x * 32 + lane;
-  float acc[K + 1];
-#pragma unroll
-  for (int k = 0; k <= K; ++k) acc[k] = 0.f;
-  if (ch < C) {
-    const long long rows = static_cast<long long>(B) * L;
-    for (long long r = wy; r < rows; r += 8) {
-      const int t = static_cast<int>(r % L);
-      const float d = du[r * C + ch];
-      acc[K] += d;
-#pragma unroll
-      for (int k = 0; k < K; ++k) {
-        const int tt = t - (K - 1) + k;
-        if (tt >= 0) acc[k] = fmaf(d, x[(r + tt - t) * C + ch], acc[k]);
-      }
-    }
-  }
-#pragma unroll
-  for (int k = 0; k <= K; ++k) part[wy][lane][k] = acc[k];
-  __syncthreads();
-  if (wy == 0 && ch < C) {
-#pragma unroll
-    for (int k = 0; k <= K; ++k) {
-      float s = 0.f;
-      for (int j = 0; j < 8; ++j) s += part[j][lane][k];
-      if (k < K) dw[ch * K + k] = s; else if (dbias != nullptr) dbias[ch] = s;
-    }
-  }
-}
-
 }  // namespace ssd
 }  // namespace recml
 
@@ -323,45 +238,5 @@ extern "C" int recml_ssd_scan(const ScanParams* p, int backward, cudaStream_t st
     default: RECML_SSD(32); break;
   }
 #undef RECML_SSD
-  return cudaGetLastError() == cudaSuccess ? 0 : -1;
-}
-
-static int conv_blocks(long long total) {
-  long long b = (total + 255) / 256;
-  return static_cast<int>(b < 1 ? 1 : (b > 148 * 16 ? 148 * 16 : b));
-}
-
-extern "C" int recml_conv1d_silu_fwd(const float* x, const float* w, const float* bias, float* y, int B, int L, int C,
-                                     int K, cudaStream_t stream) {
-  const long long total = static_cast<long long>(B) * L * C;
-  if (total == 0) return 0;
-  switch (K) {
-    case 2: conv_fwd_kernel<2><<<conv_blocks(total), 256, 0, stream>>>(x, w, bias, y, B, L, C); break;
-    case 3: conv_fwd_kernel<3><<<conv_blocks(total), 256, 0, stream>>>(x, w, bias, y, B, L, C); break;
-    case 4: conv_fwd_kernel<4><<<conv_blocks(total), 256, 0, stream>>>(x, w, bias, y, B, L, C); break;
-    default: return -10;
-  }
-  return cudaGetLastError() == cudaSuccess ? 0 : -1;
-}
-
-// du is a [B, L, C] scratch the caller provides; dbias may be null.
-extern "C" int recml_conv1d_silu_bwd(const float* x, const float* w, const float* bias, const float* dy, float* dx,
-                                     float* du, float* dw, float* dbias, int B, int L, int C, int K,
-                                     cudaStream_t stream) {
-  const long long total = static_cast<long long>(B) * L * C;
-  if (total == 0) return 0;
-  const int cb = (C + 31) / 32;
-  switch (K) {
-#define RECML_CONV(KK)                                                                              \
-    case KK:                                                                                        \
-      conv_bwd_dx_kernel<KK><<<conv_blocks(total), 256, 0, stream>>>(x, w, bias, dy, dx, du, B, L, C); \
-      conv_bwd_dw_kernel<KK><<<cb, 256, 0, stream>>>(x, du, dw, dbias, B, L, C);                    \
-      break;
-    RECML_CONV(2)
-    RECML_CONV(3)
-    RECML_CONV(4)
-#undef RECML_CONV
-    default: return -10;
-  }
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }

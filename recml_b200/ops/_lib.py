@@ -26,7 +26,7 @@ _KERNELS_PER_CALL = {"recml_emb_bwd_update": 2, "recml_allreduce_bucket": 3, "re
                      "recml_radix_sort_passes": 0, "recml_id_unique_scratch_words": 0, "recml_id_unique_sorted": 3,
                      "recml_emb_bucketize_struct_size": 0,
                      "recml_emb_struct_sizes": 0, "recml_optim_struct_sizes": 0, "recml_ar_struct_sizes": 0,
-                     "recml_ssd_struct_size": 0, "recml_ssd_ckpt_interval": 0, "recml_conv1d_silu_bwd": 2,
+                     "recml_ssd_struct_size": 0, "recml_ssd_ckpt_interval": 0,
                      "recml_hstu_struct_size": 0, "recml_vocab_rank_struct_size": 0}
 
 

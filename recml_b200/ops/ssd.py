@@ -260,36 +260,42 @@ def ssd_scan_recurrent_kernel(x, a, b, c, initial_states=None):
 
 
 class _ConvFn(torch.autograd.Function):
+  """`csrc/cuda/conv1d.cu`: rows stay in their own type (bf16 or fp32), taps and sums are fp32."""
+
   @staticmethod
   def forward(ctx, x, weight, bias):
     from recml_b200.ops import _lib
-    lib = _lib.cuda()
     B, L, C = x.shape
-    xf, wf = x.float().contiguous(), weight.float().contiguous()
+    xr, wf = _conv_rows(x).contiguous(), weight.float().contiguous()
     bf = None if bias is None else bias.float().contiguous()
-    y = torch.empty_like(xf)
-    _lib.check_rc(lib.recml_conv1d_silu_fwd(_lib.ptr(xf), _lib.ptr(wf), None if bf is None else _lib.ptr(bf), _lib.ptr(y),
-                                            ctypes.c_int(B), ctypes.c_int(L), ctypes.c_int(C),
-                                            ctypes.c_int(weight.shape[1]), _lib.stream()), "conv1d_silu_fwd")
-    ctx.save_for_backward(xf, wf, bf if bf is not None else torch.empty(0, device=x.device))
+    y = torch.empty_like(xr)
+    _lib.check_rc(_lib.cuda().recml_conv1d_silu_fwd(
+        _lib.ptr(xr), _lib.ptr(wf), _lib.ptr(bf), _lib.ptr(y), ctypes.c_int(B), ctypes.c_int(L), ctypes.c_int(C),
+        ctypes.c_int(weight.shape[1]), ctypes.c_int(int(xr.dtype == torch.bfloat16)), _lib.stream()), "conv1d_silu_fwd")
+    ctx.save_for_backward(xr, wf, bf)
     ctx.meta = (x.dtype, weight.dtype, None if bias is None else bias.dtype)
     return y.to(x.dtype)
 
   @staticmethod
   def backward(ctx, dy):
     from recml_b200.ops import _lib
-    lib = _lib.cuda()
-    xf, wf, bf = ctx.saved_tensors
+    xr, wf, bf = ctx.saved_tensors
     xdt, wdt, bdt = ctx.meta
-    B, L, C = xf.shape
-    dyf = dy.float().contiguous()
-    dx, du, dw = torch.empty_like(xf), torch.empty_like(xf), torch.empty_like(wf)
-    dbias = torch.empty(C, dtype=torch.float32, device=xf.device) if bdt is not None else None
-    _lib.check_rc(lib.recml_conv1d_silu_bwd(
-        _lib.ptr(xf), _lib.ptr(wf), _lib.ptr(bf) if bdt is not None else None, _lib.ptr(dyf), _lib.ptr(dx), _lib.ptr(du),
-        _lib.ptr(dw), None if dbias is None else _lib.ptr(dbias), ctypes.c_int(B), ctypes.c_int(L), ctypes.c_int(C),
-        ctypes.c_int(wf.shape[1]), _lib.stream()), "conv1d_silu_bwd")
-    return dx.to(xdt), dw.to(wdt), None if dbias is None else dbias.to(bdt)
+    B, L, C = xr.shape
+    K = wf.shape[1]
+    g = dy.to(xr.dtype).contiguous()
+    dx = torch.empty_like(xr)
+    sums = torch.zeros(C * (K + (bdt is not None)), dtype=torch.float32, device=xr.device)     # dw, then dbias
+    dw, dbias = sums[:C * K], None if bdt is None else sums[C * K:]
+    _lib.check_rc(_lib.cuda().recml_conv1d_silu_bwd(
+        _lib.ptr(xr), _lib.ptr(wf), _lib.ptr(bf), _lib.ptr(g), _lib.ptr(dx), _lib.ptr(dw), _lib.ptr(dbias),
+        ctypes.c_int(B), ctypes.c_int(L), ctypes.c_int(C), ctypes.c_int(K), ctypes.c_int(int(xr.dtype == torch.bfloat16)),
+        _lib.stream()), "conv1d_silu_bwd")
+    return dx.to(xdt), dw.view(C, K).to(wdt), None if dbias is None else dbias.to(bdt)
+
+
+def _conv_rows(x: torch.Tensor) -> torch.Tensor:
+  return x if x.dtype in (torch.bfloat16, torch.float32) else x.float()
 
 
 def conv1d_silu(x, weight, bias=None):

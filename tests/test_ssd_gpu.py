@@ -92,6 +92,27 @@ def test_conv_silu_matches_torch(K, use_bias):
     torch.testing.assert_close(u.grad, v.grad, rtol=1e-4, atol=1e-4)
 
 
+@pytest.mark.parametrize("B,L,C,dtype", [(2, 31, 128, torch.float32), (3, 33, 132, torch.bfloat16), (1, 1, 4, torch.bfloat16),
+                                         (2, 65, 83, torch.bfloat16), (40, 200, 640, torch.bfloat16), (1, 2, 3, torch.float32)])
+def test_conv_silu_segments_and_row_types(B, L, C, dtype):
+  """Segment edges (32 steps), one-channel rows, several blocks per channel range.  Outputs and dx carry one rounding
+  to the row type (2^-8 relative for bf16); dw sums B * L products of magnitude ~1 in fp32."""
+  torch.manual_seed(3)
+  x = torch.randn(B, L, C, device="cuda").to(dtype)
+  w, bias = torch.randn(C, 4, device="cuda") * 0.5, torch.randn(C, device="cuda") * 0.1
+  a = [t.clone().requires_grad_() for t in (x, w, bias)]
+  r = [t.float().clone().requires_grad_() for t in (x, w, bias)]
+  y, y_ref = ssd.conv1d_silu(*a), ssd.causal_depthwise_conv1d_silu(*r)
+  eps = 2.0 ** -8 if dtype == torch.bfloat16 else 1e-5
+  torch.testing.assert_close(y.float(), y_ref, rtol=eps, atol=1e-5)
+  g = torch.randn_like(y)
+  y.backward(g)
+  y_ref.backward(g.float())
+  torch.testing.assert_close(a[0].grad.float(), r[0].grad, rtol=eps, atol=2e-5)
+  for u, v in zip(a[1:], r[1:]):
+    torch.testing.assert_close(u.grad, v.grad, rtol=1e-4, atol=1e-6 * B * L + 1e-5)
+
+
 def test_mamba4rec_trains_on_gpu():
   from recml_b200.layers import mamba
   torch.manual_seed(0)
