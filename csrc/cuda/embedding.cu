@@ -914,12 +914,12 @@ struct BwdParams {
   long long val_scale;
   float* table; float* slot0; float* slot1; int dloc;
   int opt; float hp[6]; float grad_scale; int slot1_rowwise;
-  float* scratch;               // [>= ceil(n / kRange), dloc] partial sums of runs that cross range boundaries (kept zero)
+  float* scratch;               // [>= ceil(n / range_len), dloc] partial sums of runs that cross range boundaries (kept zero)
   const unsigned long long* wait_flags; int W; SeqRef seq; int* status;
   const float* hp_dev;          // non-null: the six hyper-parameters are read from device memory (so that a
                                 // captured CUDA graph follows a learning-rate schedule) instead of `hp`
   unsigned int n_cap;           // >0: *n_occ is clamped to this (capacity of the occurrence list)
-  int reserved;
+  int range_len;                // occurrences per warp and scratch line: 8, 16, .. kRange (0: kRange)
 };
 
 __device__ __forceinline__ float hpv(const BwdParams& p, int i) {
@@ -930,12 +930,17 @@ __device__ __forceinline__ unsigned int occ_count_of(const BwdParams& p) {
   return p.n_cap > 0 && n > p.n_cap ? p.n_cap : n;
 }
 
-template <int VPL>
-__device__ __forceinline__ void apply_row_update(const BwdParams& p, unsigned int row, Vec<VPL> g, int lane,
-                                                 bool lane_on) {
+// The one optimizer value per row of the row-wise optimizers (null for the others).
+__device__ __forceinline__ float* row_slot(const BwdParams& p, int opt) {
+  return opt == kRowAdagrad ? p.slot0 : opt == kRowAdam ? p.slot1 : nullptr;
+}
+
+// `w` is this lane's part of the row and `rs` its row_slot value, both loaded by the caller.  OPT: the optimizer
+// when it is known at compile time, -1 to read it from the parameters.
+template <int VPL, int OPT>
+__device__ __forceinline__ void apply_row_update(const BwdParams& p, unsigned int row, Vec<VPL> g, Vec<VPL> w, float rs,
+                                                 int lane, bool lane_on) {
   const size_t off = static_cast<size_t>(row) * p.dloc + lane * VPL;
-  Vec<VPL> w;
-  if (lane_on) w = load_f32_rw<VPL>(p.table + off);
 #pragma unroll
   for (int e = 0; e < VPL; ++e) g.v[e] *= p.grad_scale;
   float sq = 0.f;
@@ -944,7 +949,8 @@ __device__ __forceinline__ void apply_row_update(const BwdParams& p, unsigned in
     for (int e = 0; e < VPL; ++e) sq += g.v[e] * g.v[e];
   }
   const float lr = hpv(p, 0);
-  switch (p.opt) {
+  const int opt = OPT >= 0 ? OPT : p.opt;
+  switch (opt) {
     case kSGD:
       if (lane_on) {
 #pragma unroll
@@ -953,8 +959,7 @@ __device__ __forceinline__ void apply_row_update(const BwdParams& p, unsigned in
       break;
     case kRowAdagrad: {
       const float msq = warp_sum(sq) / p.dloc;
-      const float s = p.slot0[row] + msq;
-      __syncwarp();
+      const float s = rs + msq;
       if (lane == 0) p.slot0[row] = s;
       const float inv = lr / (sqrtf(s) + hpv(p, 1));
       if (lane_on) {
@@ -977,9 +982,7 @@ __device__ __forceinline__ void apply_row_update(const BwdParams& p, unsigned in
       float vrow = 0.f;
       if (p.opt == kRowAdam) {
         const float msq = warp_sum(sq) / p.dloc;
-        vrow = p.slot1[row];
-        vrow += (1.f - b2) * (msq - vrow);
-        __syncwarp();
+        vrow = rs + (1.f - b2) * (msq - rs);
         if (lane == 0) p.slot1[row] = vrow;
       }
       if (lane_on) {
@@ -1064,39 +1067,54 @@ __device__ __forceinline__ unsigned int lower_bound(const uint32_t* keys, unsign
   return lo;
 }
 
-// One warp per RANGE of kRange sorted occurrences, walked in 32-wide windows with the running sum
+// One warp per RANGE of range_len sorted occurrences, walked in 32-wide windows with the running sum
 // carried across windows; a persistent grid strides over the ranges.  A run of equal rows that lies
 // inside the range is reduced in registers and applied at once; the pieces of a run that crosses
 // range boundaries are added (fp32 atomics) into the scratch line of the range where the run STARTS,
 // and emb_bwd_finalize applies those afterwards.  Hot rows (Zipf heads with 10^5 occurrences) are
-// thereby reduced by thousands of warps in parallel, with one atomic line update per kRange
+// thereby reduced by thousands of warps in parallel, with one atomic line update per range_len
 // occurrences.
 //
 // The kernel is bound by memory latency (random 256-byte gradient vectors, random table rows), so
 // every window first asks L2 for what the NEXT window will read (its gradient vectors) and for the
 // table rows and optimizer slots of the runs that end in THIS window; the loads that follow then wait
-// for L2, not DRAM.  It uses no shared memory and at most 64 registers so that it can share the SMs with a
+// for L2, not DRAM.  A warp is still a serial chain of row updates, and what a link of that chain costs decides the
+// kernel: the row of the NEXT run end is therefore in registers before the current one is applied, and the
+// row-wise optimizer values of a window come in one gather, lane l holding that of the run that ends at entry l.
+// (Jagged bags of 8 x 16384, 1.57 M occurrences of 64 columns, lookup and update: 759 -> 684 us on a B200.)
+// The length of the chain is bounded by the range: 128 occurrences where that leaves every resident warp work,
+// down to 8 where it does not (the caller's rule).
+// It uses no shared memory and at most 64 registers so that it can share the SMs with a
 // tensor-core GEMM running on another stream: beside this library's GEMM CTA (320 threads x 104 registers,
 // ~210 KB of shared memory) an SM was measured to take three 128-thread blocks of 64 registers, but not
 // three of 80 (`blocks_per_sm` caps the grid accordingly).
 constexpr unsigned int kRange = 128;
 constexpr int kBwdThreads = 128;
 
+__host__ __device__ __forceinline__ unsigned int range_of(const BwdParams& p) {
+  return p.range_len > 0 ? static_cast<unsigned int>(p.range_len) : kRange;
+}
+
 // At most 64 registers: three blocks then share an SM with a GEMM CTA.  (A 56-register build, one allocation unit of
 // 256 registers per warp less, lets four blocks in; it measured the same step time and is not kept.)
-template <int VPL, bool GAINS>
+// OPT as in apply_row_update: with every optimizer in the body (unrolled over a batch of gradients) the 64 registers do
+// not hold the preloaded row, so the row-wise Adagrad of the recommenders has its own instance and only that one
+// loads ahead.
+template <int VPL, bool GAINS, int OPT>
 __global__ void __launch_bounds__(kBwdThreads, 8) emb_bwd_update_kernel(const BwdParams p) {
   if (p.wait_flags != nullptr && !wait_all_sources(p.wait_flags, p.W, seq_of(p.seq), p.status, 2)) return;
   const int lane = threadIdx.x & 31;
   const unsigned int n = occ_count_of(p);
   const unsigned int warps = (gridDim.x * blockDim.x) >> 5;
+  const unsigned int len = range_of(p);
   const bool lane_on = lane * VPL < p.dloc;
   const int grad_bytes = p.dloc * 2, row_bytes = p.dloc * 4;
-  const bool slot0_row = p.opt == kRowAdagrad, slot1_row = p.opt == kRowAdam;
+  const float* rslot = row_slot(p, OPT >= 0 ? OPT : p.opt);
   constexpr int kBatch = VPL <= 4 ? 8 : 4;
-  for (unsigned int range = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; range * kRange < n; range += warps) {
-    const unsigned int start = range * kRange;
-    const unsigned int end = min(start + kRange, n);
+  constexpr bool kAhead = OPT >= 0;
+  for (unsigned int range = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; range * len < n; range += warps) {
+    const unsigned int start = range * len;
+    const unsigned int end = min(start + len, n);
     const bool has_prev = start > 0, has_next = end < n;
     const uint32_t prev_key = has_prev ? p.keys[start - 1] : 0;
     const uint32_t next_key = has_next ? p.keys[end] : 0;
@@ -1130,16 +1148,25 @@ __global__ void __launch_bounds__(kBwdThreads, 8) emb_bwd_update_kernel(const Bw
       uint32_t knext = __shfl_down_sync(0xffffffffu, key, 1);
       if (lane == cnt - 1) knext = after;
       const bool ends_run = lane < cnt && ((window_is_last && lane == cnt - 1) || knext != key);
-      const unsigned int last_mask = __ballot_sync(0xffffffffu, ends_run);
+      unsigned int last_mask = __ballot_sync(0xffffffffu, ends_run);      // run ends not yet reached
+      float rs = 0.f;
       if (ends_run) {
         prefetch_l2(p.table + static_cast<size_t>(key) * p.dloc, row_bytes);
-        if (p.slot0 != nullptr) {
-          if (slot0_row) prefetch_l2(p.slot0 + key, 4); else prefetch_l2(p.slot0 + static_cast<size_t>(key) * p.dloc, row_bytes);
-        }
-        if (p.slot1 != nullptr) {
-          if (slot1_row) prefetch_l2(p.slot1 + key, 4); else prefetch_l2(p.slot1 + static_cast<size_t>(key) * p.dloc, row_bytes);
-        }
+        if (rslot != nullptr) rs = rslot[key];
+        if (p.slot0 != nullptr && p.slot0 != rslot) prefetch_l2(p.slot0 + static_cast<size_t>(key) * p.dloc, row_bytes);
+        if (p.slot1 != nullptr && p.slot1 != rslot) prefetch_l2(p.slot1 + static_cast<size_t>(key) * p.dloc, row_bytes);
       }
+      // row of the next run end (a run inside the range is this warp's alone; the row of one that crosses is read
+      // for nothing)
+      Vec<VPL> wn;
+      uint32_t kn = 0;
+      auto load_next = [&]() {
+        if (last_mask != 0) {
+          kn = __shfl_sync(0xffffffffu, key, __ffs(last_mask) - 1);
+          if (lane_on) wn = load_f32_rw<VPL>(p.table + static_cast<size_t>(kn) * p.dloc + lane * VPL);
+        }
+      };
+      if (kAhead) load_next();
       for (int j0 = 0; j0 < cnt; j0 += kBatch) {
         RawBf16<VPL> g[kBatch]; float gj[kBatch];
 #pragma unroll
@@ -1156,16 +1183,20 @@ __global__ void __launch_bounds__(kBwdThreads, 8) emb_bwd_update_kernel(const Bw
           if (j >= cnt) break;
           if (lane_on) fma_raw_bf16<VPL>(acc, gj[u], g[u]);
           if (!((last_mask >> j) & 1u)) continue;
-          const uint32_t kj = __shfl_sync(0xffffffffu, key, j);
+          if (!kAhead) load_next();
+          const uint32_t kj = kn;
+          const Vec<VPL> w = wn;
+          last_mask &= ~(1u << j);
+          if (kAhead) load_next();
           const bool at_range_end = window_is_last && j == cnt - 1;
           const bool begins = !first_run || !has_prev || (prev_key != kj);
           const bool ends = !at_range_end || !has_next || (next_key != kj);
           if (begins && ends) {
-            apply_row_update<VPL>(p, kj, acc, lane, lane_on);
+            apply_row_update<VPL, OPT>(p, kj, acc, w, __shfl_sync(0xffffffffu, rs, j), lane, lane_on);
           } else {
             unsigned int slot = range;
             if (!begins) {
-              if (lane == 0) slot = lower_bound(p.keys, start, kj) / kRange;
+              if (lane == 0) slot = lower_bound(p.keys, start, kj) / len;
               slot = __shfl_sync(0xffffffffu, slot, 0);
             }
             if (lane_on) {
@@ -1188,26 +1219,31 @@ template <int VPL>
 __global__ void __launch_bounds__(256) emb_bwd_finalize_kernel(const BwdParams p) {
   const int lane = threadIdx.x & 31;
   const unsigned int n = occ_count_of(p);
+  const unsigned int len = range_of(p);
   const unsigned int range = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const unsigned int start = range * kRange;
+  const unsigned int start = range * len;
   if (start >= n) return;
-  const unsigned int last = min(start + kRange, n) - 1;
+  const unsigned int last = min(start + len, n) - 1;
   const uint32_t klast = p.keys[last];
   if (!(last + 1 < n && p.keys[last + 1] == klast)) return;            // run does not cross into the next range
   if (p.keys[start] == klast && start > 0 && p.keys[start - 1] == klast) return;  // run started earlier
   const bool lane_on = lane * VPL < p.dloc;
   float* sp = p.scratch + static_cast<size_t>(range) * p.dloc + lane * VPL;
-  Vec<VPL> acc;
+  Vec<VPL> acc, w;
 #pragma unroll
   for (int e = 0; e < VPL; ++e) acc.v[e] = 0.f;
   if (lane_on) {
     acc = load_f32_rw<VPL>(sp);
+    w = load_f32_rw<VPL>(p.table + static_cast<size_t>(klast) * p.dloc + lane * VPL);
     Vec<VPL> z;
 #pragma unroll
     for (int e = 0; e < VPL; ++e) z.v[e] = 0.f;
     store_f32<VPL>(sp, z);
   }
-  apply_row_update<VPL>(p, klast, acc, lane, lane_on);
+  const float* rslot = row_slot(p, p.opt);
+  const float rs = rslot != nullptr ? rslot[klast] : 0.f;
+  __syncwarp();         // every lane has read the slot before lane 0 rewrites it
+  apply_row_update<VPL, -1>(p, klast, acc, w, rs, lane, lane_on);
 }
 
 __global__ void tick_kernel(unsigned long long* p) { *p += 1ull; }
@@ -1302,7 +1338,9 @@ extern "C" int recml_emb_bwd_update(const BwdParams* p, long long max_occ, int g
   const int vpl = vpl_for(p->dloc);
   if (vpl == 0 || (p->dloc % vpl) != 0) return -10;
   if (max_occ <= 0) return 0;
-  const long long ranges = (max_occ + kRange - 1) / kRange;
+  const int rl = p->range_len;
+  if (rl != 0 && rl != 8 && rl != 16 && rl != 32 && rl != 64 && rl != static_cast<int>(kRange)) return -10;
+  const long long ranges = (max_occ + range_of(*p) - 1) / range_of(*p);
   static int sms = 0;
   if (sms == 0) {
     int dev = 0;
@@ -1315,17 +1353,23 @@ extern "C" int recml_emb_bwd_update(const BwdParams* p, long long max_occ, int g
   const long long cap = static_cast<long long>(sms) * blocks_per_sm;
   const int blocks = static_cast<int>(want < cap ? want : cap);
   const int fin_blocks = static_cast<int>((ranges + 7) / 8);
-#define RECML_BWD(V)                                                                      \
+#define RECML_BWD_OPT(V, G, O)                                                            \
   do {                                                                                    \
     static bool configured = false;                                                       \
     if (!configured) {                                                                    \
-      recml::prefer_max_shared_carveout(emb_bwd_update_kernel<V, true>);                  \
-      recml::prefer_max_shared_carveout(emb_bwd_update_kernel<V, false>);                 \
+      recml::prefer_max_shared_carveout(emb_bwd_update_kernel<V, G, O>);                  \
       recml::prefer_max_shared_carveout(emb_bwd_finalize_kernel<V>);                      \
       configured = true;                                                                  \
     }                                                                                     \
-    if (gains) emb_bwd_update_kernel<V, true><<<blocks, kBwdThreads, 0, stream>>>(*p);    \
-    else emb_bwd_update_kernel<V, false><<<blocks, kBwdThreads, 0, stream>>>(*p);         \
+    emb_bwd_update_kernel<V, G, O><<<blocks, kBwdThreads, 0, stream>>>(*p);               \
+  } while (0)
+#define RECML_BWD(V)                                                                      \
+  do {                                                                                    \
+    if (p->opt == kRowAdagrad) {                                                          \
+      if (gains) RECML_BWD_OPT(V, true, kRowAdagrad); else RECML_BWD_OPT(V, false, kRowAdagrad); \
+    } else {                                                                              \
+      if (gains) RECML_BWD_OPT(V, true, -1); else RECML_BWD_OPT(V, false, -1);            \
+    }                                                                                     \
     emb_bwd_finalize_kernel<V><<<fin_blocks, 256, 0, stream>>>(*p);                       \
   } while (0)
   switch (vpl) {
@@ -1335,6 +1379,7 @@ extern "C" int recml_emb_bwd_update(const BwdParams* p, long long max_occ, int g
     default: RECML_BWD(8); break;
   }
 #undef RECML_BWD
+#undef RECML_BWD_OPT
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
@@ -1431,6 +1476,7 @@ extern "C" int recml_emb_bwd_update_static(const BwdParams* p, long long max_occ
   }
   BwdParams q = *p;
   q.scratch = scratch;
+  q.range_len = 0;
   const int rc = recml_emb_bwd_update(&q, max_occ, gains, 0, stream);
   if (rc != 0) static_fail(err, err_len, "kernel launch failed");
   return rc;

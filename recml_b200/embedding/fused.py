@@ -89,7 +89,7 @@ class BwdParams(ctypes.Structure):
               ("table", c_vp), ("slot0", c_vp), ("slot1", c_vp), ("dloc", c_int), ("opt", c_int),
               ("hp", c_float * 6), ("grad_scale", c_float), ("slot1_rowwise", c_int), ("scratch", c_vp),
               ("wait_flags", c_vp), ("W", c_int), ("seq", SeqRef), ("status", c_vp), ("hp_dev", c_vp),
-              ("n_cap", c_uint), ("reserved", c_int)]
+              ("n_cap", c_uint), ("range_len", c_int)]
 
 
 class PushIdsParams(ctypes.Structure):
@@ -131,6 +131,16 @@ def _device_struct_array(items, device) -> torch.Tensor:
     return torch.zeros(8, dtype=torch.uint8, device=device)
   raw = b"".join(bytes(x) for x in items)
   return torch.frombuffer(bytearray(raw), dtype=torch.uint8).to(device)
+
+
+def update_range(cap: int) -> int:
+  """Sorted occurrences per warp of the update kernel (a power of two, 8 to 128) for a list of `cap` entries: a warp's
+  range is a serial chain of row updates, so short lists are cut finer until the 4736 warps that are resident on a
+  GPU (148 SMs x 32) have one range each."""
+  n = 128
+  while n > 8 and cap < n * 4736:
+    n //= 2
+  return n
 
 
 class FusedBackend:
@@ -447,7 +457,8 @@ class FusedBackend:
                            count=torch.zeros(1, dtype=torch.int32, device=dev), sorted=0)
                       for _ in range(self.pipeline_depth)]
       dloc = m.plan.stacks[si].dim
-      info["scratch"] = torch.zeros((cap + 127) // 128, dloc, dtype=torch.float32, device=dev)
+      info["range_len"] = update_range(cap)
+      info["scratch"] = torch.zeros(-(-cap // info["range_len"]), dloc, dtype=torch.float32, device=dev)
       words = int(self.lib.recml_radix_sort_scratch_words(c_ll(cap)))
       info["sort_scratch"] = torch.empty(words, dtype=torch.int32, device=dev)
       info["key_bits"] = max(1, int(max(m.plan.stacks[si].rows, 1) - 1).bit_length())
@@ -691,7 +702,7 @@ class FusedBackend:
       bp.wait_flags = self._flag_ptr(m.rank, gchan, 0) if (W > 1 and direct is None) else None
       bp.W, bp.seq, bp.status = W, seq, self.status.data_ptr()
       bp.hp_dev = self._hp_dev[si].data_ptr()
-      bp.n_cap = n
+      bp.n_cap, bp.range_len = n, info["range_len"]
       if n > 0 or W > 1:
         _lib.check_rc(self.lib.recml_emb_bwd_update(ctypes.byref(bp), c_ll(max(n, 1)), c_int(int(self.has_gains)),
                                                     c_int(self.bwd_blocks_per_sm), st), "emb_bwd_update")

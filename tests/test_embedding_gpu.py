@@ -159,3 +159,48 @@ def test_id_dropping_counts_overflow_instead_of_failing():
       with pytest.raises(_lib.DeviceStatusError):
         _lib.check_status(dev)
       _lib.check_status(dev)
+
+
+@pytest.mark.parametrize("dim", [24, 64, 128, 256])
+@pytest.mark.parametrize("opt", ["rowwise_adagrad", "adagrad"])
+@pytest.mark.parametrize("range_len", [8, 16, 32, 64, 128])
+def test_update_ranges(range_len, opt, dim):
+  """The update kernel at every range length: runs that end on, before and behind range and window edges, one run over
+  many ranges, lists shorter than a range, against float64."""
+  import ctypes
+  from recml_b200.embedding import fused
+  lib, dev, rows, n_vec = _lib.cuda(), torch.device("cuda"), 400, 96
+  rng = np.random.default_rng(range_len + dim)
+  for n in (1, range_len - 1, range_len, range_len + 1, 33, 1000, 2049):
+    runs = [1, 2, range_len - 1, range_len, range_len + 1, 31, 32, 33, 3 * range_len, 1, 1, 5]
+    keys = np.concatenate([np.full(r, 2 * k) for k, r in enumerate(runs)] + [rng.integers(30, rows, n)])
+    keys = np.sort(keys)[:n].astype(np.int32)
+    vals = rng.integers(0, n_vec, n).astype(np.int32)
+    grads = (torch.randn(n_vec, dim, generator=torch.Generator().manual_seed(n)) * 0.1).to(torch.bfloat16)
+    table = torch.randn(rows, dim, generator=torch.Generator().manual_seed(1))
+    slot = torch.full((rows,) if opt == "rowwise_adagrad" else (rows, dim), 0.1)
+    t, s, g = table.to(dev), slot.to(dev), grads.to(dev)
+    k, v = torch.from_numpy(keys).to(dev), torch.from_numpy(vals).to(dev)
+    count = torch.tensor([n], dtype=torch.int32, device=dev)
+    scratch = torch.zeros(-(-n // range_len), dim, device=dev)
+    bp = fused.BwdParams()
+    bp.keys, bp.vals, bp.n_occ, bp.grads, bp.val_scale = k.data_ptr(), v.data_ptr(), count.data_ptr(), g.data_ptr(), dim
+    bp.table, bp.slot0, bp.dloc, bp.opt = t.data_ptr(), s.data_ptr(), dim, fused.OPT[opt]
+    bp.hp[0], bp.hp[1], bp.grad_scale, bp.scratch, bp.W = 0.05, 0.0, 1.0, scratch.data_ptr(), 1
+    bp.status, bp.n_cap, bp.range_len = _lib.status_buffer(dev).data_ptr(), n, range_len
+    assert lib.recml_emb_bwd_update(ctypes.byref(bp), ctypes.c_longlong(n), ctypes.c_int(0), ctypes.c_int(0), _lib.stream()) == 0
+    torch.cuda.synchronize()
+    assert float(scratch.abs().max()) == 0.0
+    occ = grads.double()[torch.from_numpy(vals).long()]
+    kl = torch.from_numpy(keys).long()
+    sums = torch.zeros(rows, dim, dtype=torch.float64).index_add_(0, kl, occ)
+    mags = torch.zeros(rows, dim, dtype=torch.float64).index_add_(0, kl, occ.abs())
+    cnt = torch.zeros(rows, dtype=torch.float64).index_add_(0, kl, torch.ones(n, dtype=torch.float64))[:, None]
+    sq = (sums ** 2).mean(-1, keepdim=True) if opt == "rowwise_adagrad" else sums ** 2
+    den = (0.1 + sq).sqrt()
+    want = torch.where(cnt > 0, table.double() - 0.05 * sums / den, table.double())
+    # an fp32 sum of m terms is off by at most m 2^-24 sum|g|; that error reaches the row once through g and once
+    # through the accumulator, each time divided by a root that is at least sqrt(0.1); a few roundings come on top
+    sum_err = cnt * 2.0 ** -24 * mags.amax(-1, keepdim=True)
+    bound = 0.05 * 2 * sum_err / 0.1 ** 0.5 + 8 * 2.0 ** -24 * (table.double().abs() + 1.0)
+    assert bool(((t.cpu().double() - want).abs() <= bound).all())
