@@ -39,10 +39,10 @@ class MultiHeadAttention(nn.Module):
     lets the op use the packed-sequence kernels instead of a dense `[B, L, L]` mask."""
     B, L, D = x.shape
     qkv = dense_ops.linear(x, self.qkv, self.qkv_bias).reshape(B, L, 3, self.num_heads, self.head_dim)
-    q, k, v = qkv.unbind(dim=2)
     if structured:
-      a = sm_ops.structured_attention(q, k, v, padding_mask, causal, self.dropout_p, self.training)
+      a = sm_ops.structured_attention_qkv(qkv, padding_mask, causal, self.dropout_p, self.training)
     else:
+      q, k, v = qkv.unbind(dim=2)
       a = sm_ops.softmax_attention(q, k, v, mask, self.dropout_p, self.training)
     return dense_ops.linear(a.reshape(B, L, D), self.out, self.out_bias)
 
@@ -66,8 +66,9 @@ class TransformerBlock(nn.Module):
 
   def forward(self, x, padding_mask=None, attention_mask=None):
     B, L, _ = x.shape
-    mask = sm_ops.merge_masks(B, L, x.device, padding_mask=padding_mask, attention_mask=attention_mask,
-                              causal=self.causal)
+    # (without an explicit attention mask the op works from padding and causality alone)
+    mask = None if attention_mask is None else sm_ops.merge_masks(
+        B, L, x.device, padding_mask=padding_mask, attention_mask=attention_mask, causal=self.causal)
     ln = norm_ops.layer_norm
     kw = dict(padding_mask=padding_mask, causal=self.causal, structured=attention_mask is None)
     if self.normalize_first:

@@ -384,10 +384,12 @@ def softmax_forward(q, k, v, seq_offsets, max_seq_len, causal, scale, dropout=No
   return out, lse
 
 
-def softmax_backward(do, out, lse, q, k, v, seq_offsets, max_seq_len, causal, scale, dropout=None):
+def softmax_backward(do, out, lse, q, k, v, seq_offsets, max_seq_len, causal, scale, dropout=None, dq_fp32: bool = False):
+  """Gradients w.r.t. q, k, v; `dq_fp32` returns dq as the kernel accumulated it."""
+  from recml_b200.ops import seq_pack
   tiles = _tiles(seq_offsets, q.shape[0], backward=True)
   do = as_rows(do)
-  delta = (do.float() * out.float()).sum(-1).contiguous()          # [T, H]
+  delta = seq_pack.head_dot(do, out)                               # [T, H]
   dq = torch.zeros(q.shape, dtype=torch.float32, device=q.device)
   dk, dv = (torch.empty(k.shape, dtype=k.dtype, device=k.device) for _ in range(2))
   p = _params(q, seq_offsets, None, None, None, max_seq_len, causal, scale, tiles, k, v, do)
@@ -396,7 +398,7 @@ def softmax_backward(do, out, lse, q, k, v, seq_offsets, max_seq_len, causal, sc
   _set_dropout(p, dropout, MODE_SOFTMAX_DROPOUT)
   _lib.check_rc(_lib.cuda().recml_hstu_attn_bwd(_lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(do), ctypes.byref(p),
                                                 c_int(tiles[2]), _lib.stream()), "softmax_attn_bwd")
-  return dq.to(q.dtype), dk, dv
+  return (dq if dq_fp32 else dq.to(q.dtype)), dk, dv
 
 
 # ---- decay mode: the quadratic ("attention") form of a diagonal state-space recurrence -----------------------

@@ -76,6 +76,56 @@ def _kernel_ok(q, L: int) -> bool:
   return hstu_cuda.available()
 
 
+class _PaddedSoftmaxFn(torch.autograd.Function):
+  """Softmax attention over the real tokens of a padded batch, from one `qkv [B, L, 3, H, Dh]`: q | k | v are packed as
+  one row per token, and the three gradients come back as one row per token.  Padding rows are zeros both ways."""
+
+  @staticmethod
+  def forward(ctx, qkv, padding_mask, causal, scale, dropout_p):
+    from recml_b200.ops import hstu_cuda, seq_pack
+    from recml_b200.ops.hstu_attention import _draw_dropout
+    B, L, _, H, Dh = qkv.shape
+    T, D = B * L, H * Dh
+    rows = qkv.detach().reshape(T, 3 * D).to(torch.bfloat16)
+    if padding_mask is None:
+      offs, src, dest = torch.arange(B + 1, device=qkv.device, dtype=torch.int32) * L, None, None
+      packed = rows if rows.is_contiguous() and rows.data_ptr() % 16 == 0 else rows.clone(memory_format=torch.contiguous_format)
+    else:
+      offs, src, dest = seq_pack.index(padding_mask)
+      packed = seq_pack.gather_rows(rows, src)
+    q, k, v = packed.view(T, 3, H, Dh).unbind(1)
+    drop = _draw_dropout(dropout_p, qkv.device)
+    out, lse = hstu_cuda.softmax_forward(q, k, v, offs, L, causal, scale, dropout=drop)
+    ctx.save_for_backward(packed, out, lse, offs, src, dest)
+    ctx.meta, ctx.drop, ctx.dtype = (L, causal, scale), drop, qkv.dtype
+    res = out if dest is None else seq_pack.gather_rows(out.view(T, D), dest)
+    return res.view(B, L, H, Dh).to(qkv.dtype)
+
+  @staticmethod
+  def backward(ctx, do):
+    from recml_b200.ops import hstu_cuda, seq_pack
+    packed, out, lse, offs, src, dest = ctx.saved_tensors
+    B, L, H, Dh = do.shape
+    T, D = B * L, H * Dh
+    g = do.reshape(T, D).to(torch.bfloat16)
+    if src is not None:
+      g = seq_pack.gather_rows(g, src)
+    q, k, v = packed.view(T, 3, H, Dh).unbind(1)
+    dq, dk, dv = hstu_cuda.softmax_backward(g.view(T, H, Dh), out, lse, q, k, v, offs, *ctx.meta, dropout=ctx.drop, dq_fp32=True)
+    return seq_pack.gather_qkv_grad(dq, dk, dv, dest).view(B, L, 3, H, Dh).to(ctx.dtype), None, None, None, None
+
+
+def structured_attention_qkv(qkv, padding_mask: torch.Tensor | None, causal: bool, dropout_p: float = 0.0,
+                             training: bool = False):
+  """`structured_attention` for q, k and v that lie together as `[B, L, 3, H, Dh]` (a fused projection's output)."""
+  B, L, _, H, Dh = qkv.shape
+  if not _kernel_ok(qkv, L):
+    q, k, v = qkv.unbind(2)
+    mask = merge_masks(B, L, q.device, padding_mask=padding_mask, causal=causal)
+    return softmax_attention(q, k, v, mask, dropout_p, training)
+  return _PaddedSoftmaxFn.apply(qkv, padding_mask, causal, 1.0 / math.sqrt(Dh), dropout_p if training else 0.0)
+
+
 def structured_attention(q, k, v, padding_mask: torch.Tensor | None, causal: bool, dropout_p: float = 0.0,
                          training: bool = False):
   """Attention whose mask is `key is not padding` ∧ (`key <= query` when causal): q, k, v `[B, L, H, Dh]`,
@@ -84,27 +134,10 @@ def structured_attention(q, k, v, padding_mask: torch.Tensor | None, causal: boo
   length), so no `[B, H, L, L]` score tensor is ever written; rows of padded queries come back as zeros
   (the dense formulation gives them the average of the visible values; nothing downstream reads them).
   Packing happens on the device without a host synchronisation: every real token goes to its rank among
-  the real tokens, padding goes to a spare row, and the kernels see `B * L` rows of capacity.
+  the real tokens, and the kernels see `B * L` rows of capacity.
   Everywhere else this is `softmax_attention` with the merged mask."""
-  B, L, H, Dh = q.shape
-  drop = dropout_p if training else 0.0
+  B, L = q.shape[:2]
   if not _kernel_ok(q, L):
     mask = merge_masks(B, L, q.device, padding_mask=padding_mask, causal=causal)
     return softmax_attention(q, k, v, mask, dropout_p, training)
-  dt = q.dtype
-  flat = lambda t: t.reshape(B * L, H, Dh).to(torch.bfloat16)
-  if padding_mask is None:
-    offs = torch.arange(B + 1, device=q.device, dtype=torch.int32) * L
-    out = jagged_softmax_attention(flat(q), flat(k), flat(v), offs, L, causal, dropout_p=drop)
-    return out.reshape(B, L, H, Dh).to(dt)
-  T = B * L
-  valid = padding_mask.bool().reshape(T)
-  rank = torch.cumsum(valid, 0, dtype=torch.int32) - 1
-  dest = torch.where(valid, rank, torch.full_like(rank, T)).long()       # padding lands in the spare row T
-  offs = torch.zeros(B + 1, dtype=torch.int32, device=q.device)
-  offs[1:] = valid.reshape(B, L).sum(1).cumsum(0)
-  pack = lambda t: torch.zeros(T + 1, H, Dh, dtype=torch.bfloat16, device=q.device).index_copy(0, dest, flat(t))[:T]
-  packed = jagged_softmax_attention(pack(q), pack(k), pack(v), offs, L, causal, dropout_p=drop)
-  # (rows past the last real token are never written by the kernels: select, do not multiply)
-  out = torch.where(valid[:, None, None], packed.index_select(0, dest.clamp(max=T - 1)), torch.zeros((), dtype=packed.dtype, device=q.device))
-  return out.reshape(B, L, H, Dh).to(dt)
+  return structured_attention_qkv(torch.stack((q, k, v), dim=2), padding_mask, causal, dropout_p, training).to(q.dtype)
