@@ -35,8 +35,12 @@ class SASRecRetrieval(nn.Module):
 
   def _lookup(self, a, b, c):
     B, L = a.shape
-    kjt = emb.KeyedJagged.from_dense({"input": a.reshape(-1, 1), "positive": b.reshape(-1, 1),
-                                      "negative": c.reshape(-1, 1)}).to_device(a.device)
+    ids = {"input": a, "positive": b, "negative": c}
+    if a.is_cuda:       # one id per bag: the offsets are made where the ids are
+      kjt = emb.KeyedJagged(tuple(ids), torch.cat([t.reshape(-1).to(torch.int32) for t in ids.values()]),
+                            torch.arange(3 * B * L + 1, dtype=torch.int32, device=a.device), None, B * L)
+    else:
+      kjt = emb.KeyedJagged.from_dense({k: t.reshape(-1, 1) for k, t in ids.items()}).to_device(a.device)
     out = self.items(kjt)                       # [B·L, 3, D]
     return out.view(B, L, 3, self.model_dim).unbind(dim=2)
 
