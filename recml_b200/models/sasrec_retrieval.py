@@ -8,6 +8,7 @@ from torch import nn
 
 from recml_b200 import embedding as emb
 from recml_b200.layers import sasrec as sasrec_layers
+from recml_b200.ops import pair_loss
 from recml_b200.ops import vocab_rank
 
 
@@ -47,11 +48,8 @@ class SASRecRetrieval(nn.Module):
   def forward(self, input_ids, positive_ids, negative_ids, padding_mask):
     """All `[B, L]`.  Returns the masked mean BCE over positions."""
     e_in, e_pos, e_neg = self._lookup(input_ids, positive_ids, negative_ids)
-    h = self.encoder.encode_embeddings(e_in, padding_mask).float()
-    pos, neg = (h * e_pos.float()).sum(-1), (h * e_neg.float()).sum(-1)
-    w = padding_mask.float()
-    loss = (torch.nn.functional.softplus(-pos) + torch.nn.functional.softplus(neg)) * w
-    return loss.sum() / w.sum().clamp_min(1.0)
+    h = self.encoder.encode_embeddings(e_in, padding_mask)
+    return pair_loss.pair_bce(h, e_pos, e_neg, padding_mask)
 
   @torch.no_grad()
   def item_shard_bf16(self):
