@@ -147,11 +147,13 @@ __device__ __forceinline__ void store_bf16(__nv_bfloat16* p, const Vec<VPL>& r) 
   }
 }
 
-__device__ __forceinline__ float warp_sum(float x) {
+template <int G>
+__device__ __forceinline__ float group_sum(float x) {      // over G neighbouring lanes (all 32 take part)
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+  for (int o = G / 2; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
   return x;
 }
+__device__ __forceinline__ float warp_sum(float x) { return group_sum<32>(x); }
 
 // Asks L2 for the 128-byte lines of [ptr, ptr + bytes): issued a window ahead of the loads that need them, so
 // those loads pay the L2 latency instead of the DRAM one.
@@ -931,13 +933,12 @@ __device__ __forceinline__ unsigned int occ_count_of(const BwdParams& p) {
 }
 
 // The one optimizer value per row of the row-wise optimizers (null for the others).
-__device__ __forceinline__ float* row_slot(const BwdParams& p, int opt) {
-  return opt == kRowAdagrad ? p.slot0 : opt == kRowAdam ? p.slot1 : nullptr;
+__device__ __forceinline__ float* row_slot(const BwdParams& p) {
+  return p.opt == kRowAdagrad ? p.slot0 : p.opt == kRowAdam ? p.slot1 : nullptr;
 }
 
-// `w` is this lane's part of the row and `rs` its row_slot value, both loaded by the caller.  OPT: the optimizer
-// when it is known at compile time, -1 to read it from the parameters.
-template <int VPL, int OPT>
+// `w` is this lane's part of the row and `rs` its row_slot value, both loaded by the caller.
+template <int VPL>
 __device__ __forceinline__ void apply_row_update(const BwdParams& p, unsigned int row, Vec<VPL> g, Vec<VPL> w, float rs,
                                                  int lane, bool lane_on) {
   const size_t off = static_cast<size_t>(row) * p.dloc + lane * VPL;
@@ -949,8 +950,7 @@ __device__ __forceinline__ void apply_row_update(const BwdParams& p, unsigned in
     for (int e = 0; e < VPL; ++e) sq += g.v[e] * g.v[e];
   }
   const float lr = hpv(p, 0);
-  const int opt = OPT >= 0 ? OPT : p.opt;
-  switch (opt) {
+  switch (p.opt) {
     case kSGD:
       if (lane_on) {
 #pragma unroll
@@ -1057,16 +1057,6 @@ __device__ __forceinline__ void apply_row_update(const BwdParams& p, unsigned in
   if (lane_on) store_f32<VPL>(p.table + off, w);
 }
 
-// first index i in [0, hi) with keys[i] >= key  (keys sorted ascending)
-__device__ __forceinline__ unsigned int lower_bound(const uint32_t* keys, unsigned int hi, uint32_t key) {
-  unsigned int lo = 0;
-  while (lo < hi) {
-    const unsigned int mid = (lo + hi) >> 1;
-    if (keys[mid] < key) lo = mid + 1; else hi = mid;
-  }
-  return lo;
-}
-
 // One warp per RANGE of range_len sorted occurrences, walked in 32-wide windows with the running sum
 // carried across windows; a persistent grid strides over the ranges.  A run of equal rows that lies
 // inside the range is reduced in registers and applied at once; the pieces of a run that crosses
@@ -1075,16 +1065,12 @@ __device__ __forceinline__ unsigned int lower_bound(const uint32_t* keys, unsign
 // thereby reduced by thousands of warps in parallel, with one atomic line update per range_len
 // occurrences.
 //
-// The kernel is bound by memory latency (random 256-byte gradient vectors, random table rows), so
+// The kernels are bound by memory latency (random 256-byte gradient vectors, random table rows), so
 // every window first asks L2 for what the NEXT window will read (its gradient vectors) and for the
 // table rows and optimizer slots of the runs that end in THIS window; the loads that follow then wait
-// for L2, not DRAM.  A warp is still a serial chain of row updates, and what a link of that chain costs decides the
-// kernel: the row of the NEXT run end is therefore in registers before the current one is applied, and the
-// row-wise optimizer values of a window come in one gather, lane l holding that of the run that ends at entry l.
-// (Jagged bags of 8 x 16384, 1.57 M occurrences of 64 columns, lookup and update: 759 -> 684 us on a B200.)
-// The length of the chain is bounded by the range: 128 occurrences where that leaves every resident warp work,
-// down to 8 where it does not (the caller's rule).
-// It uses no shared memory and at most 64 registers so that it can share the SMs with a
+// for L2, not DRAM.  The length of a chain is bounded by the range: 128 occurrences where that leaves every resident
+// walker work, down to 8 where it does not (the caller's rule).
+// They use no shared memory and at most 64 registers so that they can share the SMs with a
 // tensor-core GEMM running on another stream: beside this library's GEMM CTA (320 threads x 104 registers,
 // ~210 KB of shared memory) an SM was measured to take three 128-thread blocks of 64 registers, but not
 // three of 80 (`blocks_per_sm` caps the grid accordingly).
@@ -1095,12 +1081,168 @@ __host__ __device__ __forceinline__ unsigned int range_of(const BwdParams& p) {
   return p.range_len > 0 ? static_cast<unsigned int>(p.range_len) : kRange;
 }
 
+// First index i in [0, hi) with keys[i] >= key (hi where there is none), found by the G lanes of a group together: G
+// probes per step instead of one, because a run over many ranges pays this chain of loads once per range.  Called by
+// the whole warp; groups with hi = 0 wait.
+template <int G>
+__device__ __forceinline__ unsigned int group_lower_bound(const uint32_t* keys, unsigned int hi, uint32_t key, int lane) {
+  const int sub = lane % G;
+  const unsigned int group_bits = G == 32 ? 0xffffffffu : (1u << (G & 31)) - 1u;
+  unsigned int lo = 0;
+  while (__any_sync(0xffffffffu, lo < hi)) {
+    const unsigned int step = (hi - lo + G - 1) / G;
+    const unsigned int pos = lo + sub * step;
+    const bool less = lo < hi && pos < hi && keys[pos] < key;
+    const int n = __popc((__ballot_sync(0xffffffffu, less) >> (lane - sub)) & group_bits);   // probes below `key`: a prefix
+    if (lo < hi) {
+      if (n == 0) {
+        hi = lo;
+      } else {
+        hi = min(hi, lo + n * step);
+        lo += (n - 1) * step + 1;
+      }
+    }
+  }
+  return lo;
+}
+
+// Row-wise Adagrad, the optimizer of the recommenders, for rows of 8 G columns at most: G lanes of eight columns walk a
+// range, so a warp walks 32 / G ranges at once (two for 128 columns).  The walkers of a warp are independent chains of
+// row updates that share their instructions, which halves (128 columns) the instructions of an occurrence and doubles
+// the loads in flight of a warp; beside a GEMM only 12 warps fit an SM.  The row of a walker's next run end is loaded
+// when the previous one has been applied, and the accumulators of a window come in one gather, lane l holding that of the run
+// that ends at entry l.  All control flow is uniform over the warp; a walker without work carries empty predicates.
+// On a B200, against one warp per range: DLRM step of 65536 samples 13.5 -> 12.2 ms (the update runs beside the
+// weight-gradient products), of 8192 samples 2.15 -> 1.98 ms; lookup and update of 1.57 M occurrences of 64 columns
+// 748 -> 582 us.
+template <int G, bool GAINS>
+__global__ void __launch_bounds__(kBwdThreads, 8) emb_bwd_rows_kernel(const BwdParams p) {
+  if (p.wait_flags != nullptr && !wait_all_sources(p.wait_flags, p.W, seq_of(p.seq), p.status, 2)) return;
+  constexpr unsigned int kAll = 0xffffffffu;
+  constexpr unsigned int kWalkers = 32 / G;
+  constexpr int kBatch = 4;
+  const int lane = threadIdx.x & 31, sub = lane % G, grp = lane / G;
+  const unsigned int group_bits = G == 32 ? kAll : (1u << (G & 31)) - 1u;
+  const unsigned int n = occ_count_of(p);
+  const unsigned int warps = (gridDim.x * blockDim.x) >> 5;
+  const unsigned int len = range_of(p);
+  const bool lane_on = sub * 8 < p.dloc;
+  const int grad_bytes = p.dloc * 2, row_bytes = p.dloc * 4;
+  const float lr = hpv(p, 0), eps = hpv(p, 1), gscale = p.grad_scale, dloc = static_cast<float>(p.dloc);
+  const unsigned int n_ranges = (n + len - 1) / len;
+  for (unsigned int r0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * kWalkers; r0 < n_ranges; r0 += warps * kWalkers) {
+    const unsigned int range = r0 + grp;
+    const unsigned int start = range < n_ranges ? range * len : n;
+    const unsigned int end = min(start + len, n);           // start == end: nothing for this walker
+    const bool has_prev = start > 0 && start < end, has_next = end < n;
+    const uint32_t prev_key = has_prev ? p.keys[start - 1] : 0;
+    const uint32_t next_key = has_next ? p.keys[end] : 0;
+    Vec<8> acc, wn;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) { acc.v[e] = 0.f; wn.v[e] = 0.f; }
+    bool first_run = true;      // no run has been closed yet: the open one may have begun before `start`
+    uint32_t key = 0xffffffffu; unsigned int gv = 0; float gain = 1.f;
+    auto fetch = [&](unsigned int w0, uint32_t& k, unsigned int& g, float& gn) {
+      k = 0xffffffffu; g = 0; gn = 1.f;
+      if (w0 + sub < end) {
+        k = p.keys[w0 + sub];
+        const uint32_t val = p.vals[w0 + sub];
+        g = val;
+        if (GAINS) {
+          g = __float_as_uint(p.occ_gain[2 * static_cast<size_t>(val)]);
+          gn = p.occ_gain[2 * static_cast<size_t>(val) + 1];
+        }
+        prefetch_l2(p.grads + static_cast<size_t>(g) * p.val_scale, grad_bytes);
+      }
+    };
+    fetch(start, key, gv, gain);
+    for (unsigned int w0 = start; __any_sync(kAll, w0 < end); w0 += G) {
+      const int cnt = w0 < end ? static_cast<int>(min(static_cast<unsigned int>(G), end - w0)) : 0;
+      const bool window_is_last = w0 + cnt >= end;
+      uint32_t nkey = 0xffffffffu; unsigned int ngv = 0; float ngain = 1.f;
+      if (!window_is_last) fetch(w0 + G, nkey, ngv, ngain);
+      const uint32_t after = __shfl_sync(kAll, nkey, 0, G);
+      uint32_t knext = __shfl_down_sync(kAll, key, 1, G);
+      if (sub == cnt - 1) knext = after;
+      // entries that end a run (the range's last entry always closes the open piece)
+      const bool ends_run = sub < cnt && ((window_is_last && sub == cnt - 1) || knext != key);
+      unsigned int mask = (__ballot_sync(kAll, ends_run) >> (lane - sub)) & group_bits;      // run ends not yet reached
+      float rs = 0.f;
+      if (ends_run) {
+        prefetch_l2(p.table + static_cast<size_t>(key) * p.dloc, row_bytes);
+        rs = p.slot0[key];
+      }
+      // row of the next run end (a run inside the range is this walker's alone; the row of one that crosses is read for
+      // nothing)
+      auto load_next = [&]() {
+        const uint32_t k = __shfl_sync(kAll, key, mask != 0 ? __ffs(mask) - 1 : 0, G);
+        if (mask != 0 && lane_on) wn = load_f32_rw<8>(p.table + static_cast<size_t>(k) * p.dloc + sub * 8);
+      };
+      load_next();
+      const int cnt_max = __reduce_max_sync(kAll, cnt);
+      for (int j0 = 0; j0 < cnt_max; j0 += kBatch) {
+        RawBf16<8> g[kBatch];
+#pragma unroll
+        for (int u = 0; u < kBatch; ++u) {
+          const unsigned int gvj = __shfl_sync(kAll, gv, j0 + u, G);
+          g[u] = RawBf16<8>{{0u, 0u, 0u, 0u}};
+          if (lane_on && j0 + u < cnt) g[u] = load_raw_bf16<8>(p.grads + static_cast<size_t>(gvj) * p.val_scale + sub * 8);
+        }
+        // entries of this batch at which some walker ends a run
+        const unsigned int some = __reduce_or_sync(kAll, mask >> j0) & ((1u << kBatch) - 1u);
+#pragma unroll
+        for (int u = 0; u < kBatch; ++u) {
+          const int j = j0 + u;
+          fma_raw_bf16<8>(acc, GAINS ? __shfl_sync(kAll, gain, j, G) : 1.f, g[u]);
+          if (!((some >> u) & 1u)) continue;
+          const bool mine = (mask >> j) & 1u;
+          const uint32_t kj = __shfl_sync(kAll, key, j, G);
+          const float rsj = __shfl_sync(kAll, rs, j, G);
+          const bool at_range_end = window_is_last && j == cnt - 1;
+          const bool begins = !first_run || !has_prev || (prev_key != kj);
+          const bool ends = !at_range_end || !has_next || (next_key != kj);
+          const bool apply = mine && begins && ends, part = mine && !apply;
+          float sq = 0.f;
+#pragma unroll
+          for (int e = 0; e < 8; ++e) { const float t = acc.v[e] * gscale; sq = fmaf(t, t, sq); }
+          const float s = rsj + group_sum<G>(lane_on ? sq : 0.f) / dloc;
+          if (apply) {
+            if (sub == 0) p.slot0[kj] = s;
+            const float inv = lr / (sqrtf(s) + eps);
+            if (lane_on) {
+#pragma unroll
+              for (int e = 0; e < 8; ++e) wn.v[e] -= inv * (acc.v[e] * gscale);
+              store_f32<8>(p.table + static_cast<size_t>(kj) * p.dloc + sub * 8, wn);
+            }
+          }
+          if (__any_sync(kAll, part)) {
+            const unsigned int first = group_lower_bound<G>(p.keys, part && !begins ? start : 0u, kj, lane);
+            if (part && lane_on) {
+              const unsigned int slot = begins ? range : first / len;
+              float4* sp = reinterpret_cast<float4*>(p.scratch + static_cast<size_t>(slot) * p.dloc + sub * 8);
+              atomicAdd(sp, make_float4(acc.v[0], acc.v[1], acc.v[2], acc.v[3]));
+              atomicAdd(sp + 1, make_float4(acc.v[4], acc.v[5], acc.v[6], acc.v[7]));
+            }
+          }
+          if (mine) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) acc.v[e] = 0.f;
+            first_run = false;
+            mask &= ~(1u << j);
+          }
+          const uint32_t kn = __shfl_sync(kAll, key, mask != 0 ? __ffs(mask) - 1 : 0, G);
+          if (mine && mask != 0 && lane_on) wn = load_f32_rw<8>(p.table + static_cast<size_t>(kn) * p.dloc + sub * 8);
+        }
+      }
+      key = nkey; gv = ngv; gain = ngain;
+    }
+  }
+}
+
+// The other optimizers, and rows that do not split into 16-byte parts: one warp per range.
 // At most 64 registers: three blocks then share an SM with a GEMM CTA.  (A 56-register build, one allocation unit of
 // 256 registers per warp less, lets four blocks in; it measured the same step time and is not kept.)
-// OPT as in apply_row_update: with every optimizer in the body (unrolled over a batch of gradients) the 64 registers do
-// not hold the preloaded row, so the row-wise Adagrad of the recommenders has its own instance and only that one
-// loads ahead.
-template <int VPL, bool GAINS, int OPT>
+template <int VPL, bool GAINS>
 __global__ void __launch_bounds__(kBwdThreads, 8) emb_bwd_update_kernel(const BwdParams p) {
   if (p.wait_flags != nullptr && !wait_all_sources(p.wait_flags, p.W, seq_of(p.seq), p.status, 2)) return;
   const int lane = threadIdx.x & 31;
@@ -1109,9 +1251,8 @@ __global__ void __launch_bounds__(kBwdThreads, 8) emb_bwd_update_kernel(const Bw
   const unsigned int len = range_of(p);
   const bool lane_on = lane * VPL < p.dloc;
   const int grad_bytes = p.dloc * 2, row_bytes = p.dloc * 4;
-  const float* rslot = row_slot(p, OPT >= 0 ? OPT : p.opt);
+  const float* rslot = row_slot(p);
   constexpr int kBatch = VPL <= 4 ? 8 : 4;
-  constexpr bool kAhead = OPT >= 0;
   for (unsigned int range = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; range * len < n; range += warps) {
     const unsigned int start = range * len;
     const unsigned int end = min(start + len, n);
@@ -1148,25 +1289,13 @@ __global__ void __launch_bounds__(kBwdThreads, 8) emb_bwd_update_kernel(const Bw
       uint32_t knext = __shfl_down_sync(0xffffffffu, key, 1);
       if (lane == cnt - 1) knext = after;
       const bool ends_run = lane < cnt && ((window_is_last && lane == cnt - 1) || knext != key);
-      unsigned int last_mask = __ballot_sync(0xffffffffu, ends_run);      // run ends not yet reached
-      float rs = 0.f;
+      const unsigned int last_mask = __ballot_sync(0xffffffffu, ends_run);
       if (ends_run) {
         prefetch_l2(p.table + static_cast<size_t>(key) * p.dloc, row_bytes);
-        if (rslot != nullptr) rs = rslot[key];
+        if (rslot != nullptr) prefetch_l2(rslot + key, 4);
         if (p.slot0 != nullptr && p.slot0 != rslot) prefetch_l2(p.slot0 + static_cast<size_t>(key) * p.dloc, row_bytes);
         if (p.slot1 != nullptr && p.slot1 != rslot) prefetch_l2(p.slot1 + static_cast<size_t>(key) * p.dloc, row_bytes);
       }
-      // row of the next run end (a run inside the range is this warp's alone; the row of one that crosses is read
-      // for nothing)
-      Vec<VPL> wn;
-      uint32_t kn = 0;
-      auto load_next = [&]() {
-        if (last_mask != 0) {
-          kn = __shfl_sync(0xffffffffu, key, __ffs(last_mask) - 1);
-          if (lane_on) wn = load_f32_rw<VPL>(p.table + static_cast<size_t>(kn) * p.dloc + lane * VPL);
-        }
-      };
-      if (kAhead) load_next();
       for (int j0 = 0; j0 < cnt; j0 += kBatch) {
         RawBf16<VPL> g[kBatch]; float gj[kBatch];
 #pragma unroll
@@ -1183,22 +1312,16 @@ __global__ void __launch_bounds__(kBwdThreads, 8) emb_bwd_update_kernel(const Bw
           if (j >= cnt) break;
           if (lane_on) fma_raw_bf16<VPL>(acc, gj[u], g[u]);
           if (!((last_mask >> j) & 1u)) continue;
-          if (!kAhead) load_next();
-          const uint32_t kj = kn;
-          const Vec<VPL> w = wn;
-          last_mask &= ~(1u << j);
-          if (kAhead) load_next();
+          const uint32_t kj = __shfl_sync(0xffffffffu, key, j);
           const bool at_range_end = window_is_last && j == cnt - 1;
           const bool begins = !first_run || !has_prev || (prev_key != kj);
           const bool ends = !at_range_end || !has_next || (next_key != kj);
           if (begins && ends) {
-            apply_row_update<VPL, OPT>(p, kj, acc, w, __shfl_sync(0xffffffffu, rs, j), lane, lane_on);
+            Vec<VPL> w;
+            if (lane_on) w = load_f32_rw<VPL>(p.table + static_cast<size_t>(kj) * p.dloc + lane * VPL);
+            apply_row_update<VPL>(p, kj, acc, w, rslot != nullptr ? rslot[kj] : 0.f, lane, lane_on);
           } else {
-            unsigned int slot = range;
-            if (!begins) {
-              if (lane == 0) slot = lower_bound(p.keys, start, kj) / len;
-              slot = __shfl_sync(0xffffffffu, slot, 0);
-            }
+            const unsigned int slot = begins ? range : group_lower_bound<32>(p.keys, start, kj, lane) / len;
             if (lane_on) {
               float* sp = p.scratch + static_cast<size_t>(slot) * p.dloc + lane * VPL;
 #pragma unroll
@@ -1240,10 +1363,10 @@ __global__ void __launch_bounds__(256) emb_bwd_finalize_kernel(const BwdParams p
     for (int e = 0; e < VPL; ++e) z.v[e] = 0.f;
     store_f32<VPL>(sp, z);
   }
-  const float* rslot = row_slot(p, p.opt);
+  const float* rslot = row_slot(p);
   const float rs = rslot != nullptr ? rslot[klast] : 0.f;
   __syncwarp();         // every lane has read the slot before lane 0 rewrites it
-  apply_row_update<VPL, -1>(p, klast, acc, w, rs, lane, lane_on);
+  apply_row_update<VPL>(p, klast, acc, w, rs, lane, lane_on);
 }
 
 __global__ void tick_kernel(unsigned long long* p) { *p += 1ull; }
@@ -1349,27 +1472,35 @@ extern "C" int recml_emb_bwd_update(const BwdParams* p, long long max_occ, int g
   }
   if (blocks_per_sm < 0) blocks_per_sm = 3;      // what fits beside a resident GEMM CTA
   if (blocks_per_sm == 0) blocks_per_sm = 8;
-  long long want = (ranges + (kBwdThreads / 32) - 1) / (kBwdThreads / 32);
+  // 16-byte parts of eight columns: gradients are bf16 vectors at multiples of val_scale elements
+  const uintptr_t ptrs = reinterpret_cast<uintptr_t>(p->grads) | reinterpret_cast<uintptr_t>(p->table) | reinterpret_cast<uintptr_t>(p->scratch);
+  const bool by_rows = p->opt == kRowAdagrad && p->dloc % 8 == 0 && p->val_scale % 8 == 0 && (ptrs & 15) == 0;
+  const int walkers = by_rows ? 8 / vpl : 1;         // ranges that a warp walks at once
+  const long long warps_wanted = (ranges + walkers - 1) / walkers;
+  long long want = (warps_wanted + (kBwdThreads / 32) - 1) / (kBwdThreads / 32);
   const long long cap = static_cast<long long>(sms) * blocks_per_sm;
   const int blocks = static_cast<int>(want < cap ? want : cap);
   const int fin_blocks = static_cast<int>((ranges + 7) / 8);
-#define RECML_BWD_OPT(V, G, O)                                                            \
+#define RECML_BWD_LAUNCH(K, ...)                                                          \
   do {                                                                                    \
     static bool configured = false;                                                       \
     if (!configured) {                                                                    \
-      recml::prefer_max_shared_carveout(emb_bwd_update_kernel<V, G, O>);                  \
-      recml::prefer_max_shared_carveout(emb_bwd_finalize_kernel<V>);                      \
+      recml::prefer_max_shared_carveout(K<__VA_ARGS__>);                                  \
       configured = true;                                                                  \
     }                                                                                     \
-    emb_bwd_update_kernel<V, G, O><<<blocks, kBwdThreads, 0, stream>>>(*p);               \
+    K<__VA_ARGS__><<<blocks, kBwdThreads, 0, stream>>>(*p);                               \
   } while (0)
 #define RECML_BWD(V)                                                                      \
   do {                                                                                    \
-    if (p->opt == kRowAdagrad) {                                                          \
-      if (gains) RECML_BWD_OPT(V, true, kRowAdagrad); else RECML_BWD_OPT(V, false, kRowAdagrad); \
+    if (by_rows) {                                                                        \
+      if (gains) RECML_BWD_LAUNCH(emb_bwd_rows_kernel, 4 * V, true);                      \
+      else RECML_BWD_LAUNCH(emb_bwd_rows_kernel, 4 * V, false);                           \
     } else {                                                                              \
-      if (gains) RECML_BWD_OPT(V, true, -1); else RECML_BWD_OPT(V, false, -1);            \
+      if (gains) RECML_BWD_LAUNCH(emb_bwd_update_kernel, V, true);                        \
+      else RECML_BWD_LAUNCH(emb_bwd_update_kernel, V, false);                             \
     }                                                                                     \
+    static bool configured = false;                                                       \
+    if (!configured) { recml::prefer_max_shared_carveout(emb_bwd_finalize_kernel<V>); configured = true; } \
     emb_bwd_finalize_kernel<V><<<fin_blocks, 256, 0, stream>>>(*p);                       \
   } while (0)
   switch (vpl) {
@@ -1379,7 +1510,7 @@ extern "C" int recml_emb_bwd_update(const BwdParams* p, long long max_occ, int g
     default: RECML_BWD(8); break;
   }
 #undef RECML_BWD
-#undef RECML_BWD_OPT
+#undef RECML_BWD_LAUNCH
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 

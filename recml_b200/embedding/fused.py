@@ -133,12 +133,12 @@ def _device_struct_array(items, device) -> torch.Tensor:
   return torch.frombuffer(bytearray(raw), dtype=torch.uint8).to(device)
 
 
-def update_range(cap: int) -> int:
-  """Sorted occurrences per warp of the update kernel (a power of two, 8 to 128) for a list of `cap` entries: a warp's
-  range is a serial chain of row updates, so short lists are cut finer until the 4736 warps that are resident on a
-  GPU (148 SMs x 32) have one range each."""
+def update_range(cap: int, walkers: int) -> int:
+  """Sorted occurrences per range of the update kernels (a power of two, 8 to 128) for a list of `cap` entries: a range
+  is a serial chain of row updates, so short lists are cut finer until the 4736 warps that are resident on a GPU
+  (148 SMs x 32), each walking `walkers` ranges, have work."""
   n = 128
-  while n > 8 and cap < n * 4736:
+  while n > 8 and cap < n * 4736 * walkers:
     n //= 2
   return n
 
@@ -457,7 +457,7 @@ class FusedBackend:
                            count=torch.zeros(1, dtype=torch.int32, device=dev), sorted=0)
                       for _ in range(self.pipeline_depth)]
       dloc = m.plan.stacks[si].dim
-      info["range_len"] = update_range(cap)
+      info["range_len"] = update_range(cap, max(1, 256 // dloc) if m.plan.stacks[si].optimizer.kind == "rowwise_adagrad" else 1)
       info["scratch"] = torch.zeros(-(-cap // info["range_len"]), dloc, dtype=torch.float32, device=dev)
       words = int(self.lib.recml_radix_sort_scratch_words(c_ll(cap)))
       info["sort_scratch"] = torch.empty(words, dtype=torch.int32, device=dev)
