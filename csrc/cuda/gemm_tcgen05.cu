@@ -195,7 +195,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     // 64-column slabs.  Per slab a warp (1) TMA-loads the 32 x 64 boxes of the auxiliary operands into
     // its private staging set, (2) reads the accumulator from tensor memory, applies the epilogue and
     // writes the bf16 results OVER the auxiliary boxes (same thread, same 16-byte chunk), (3) hands the
-    // boxes to TMA stores.  While one warp waits for its loads or for its store to drain, its sibling
+    // boxes to TMA stores.  With at most one auxiliary operand a slab needs one box, and the slabs take the
+    // set's two boxes in turn, so that a slab does not wait for the store of the one before it
+    // (HSTU training at 65 k tokens, K = 256 products: 12.92 -> 12.88 ms; SASRec evaluation 2.10 -> 2.08 ms).  While one warp waits for its loads or for its store to drain, its sibling
     // computes, so the quarter keeps a slab in flight at every stage.  All global traffic of the
     // epilogue is full 128-byte lines and only __syncwarp is needed.  fp32 outputs (weight gradients)
     // are written directly: a thread's 32 floats already are one full line.
@@ -206,6 +208,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     const uint32_t aux_bar = bars + 8u * (2 * C::kStages + 4 + quarter * 2 + sub);
     const int n_aux = p.epi == kEpiLinear ? 0 : ((p.epi == kEpiCross || ((p.epi == kEpiMulAdd || p.epi == kEpiAdd) && p.aux1 != nullptr)) ? 2 : 1);
     const bool cross = p.epi == kEpiCross;
+    const uint32_t flip = n_aux < 2 ? 4096u : 0u;
+    uint32_t box = 0;           // offset of this slab's box in the staging set
     auto slabs_of = [&](int tl) {
       const int rem = p.N - (tl % n_tiles) * BN;
       return rem >= BN ? BN / 64 : (rem + 63) / 64;
@@ -232,12 +236,14 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
 #pragma unroll 1
         for (int sl = sub; sl < n_slabs && ok; sl += 2) {
           const int col0 = n0 + sl * 64;
+          box ^= flip;
           if (lane == 0) {
-            // this warp's previous store has finished reading the staging set
-            asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+            // the store that last used this box has finished reading it
+            if (flip) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+            else asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
             if (n_aux > 0) {
               mbar_expect_tx(aux_bar, 4096u * n_aux);
-              tma_load_2d(my_smem, &map_x0, col0, row0, aux_bar);
+              tma_load_2d(my_smem + box, &map_x0, col0, row0, aux_bar);
               if (n_aux == 2) tma_load_2d(my_smem + 4096, &map_x1, col0, row0, aux_bar);
             }
           }
@@ -255,7 +261,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
 #pragma unroll
             for (int g = 0; g < 4; ++g) {
               const int col = col0 + hh * 32 + g * 8;
-              const int chunk = ((hh * 4 + g) ^ (lane & 7)) * 16 + lane * 128;
+              const int chunk = box + ((hh * 4 + g) ^ (lane & 7)) * 16 + lane * 128;
               float x[8];
 #pragma unroll
               for (int j = 0; j < 8; ++j) x[j] = __uint_as_float(r[g * 8 + j]);
@@ -332,7 +338,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
           fence_async_smem();
           __syncwarp();
           if (lane == 0) {
-            tma_store_2d(&map_d, col0, row0, my_smem + (cross ? 4096u : 0u));
+            tma_store_2d(&map_d, col0, row0, my_smem + (cross ? 4096u : box));
             if (cross && p.out2 != nullptr) tma_store_2d(&map_d2, col0, row0, my_smem);
             asm volatile("cp.async.bulk.commit_group;" ::: "memory");
           }
