@@ -14,6 +14,7 @@ from torch import nn
 from recml_b200.layers import embeddings as emb_layers
 from recml_b200.layers import utils as layer_utils
 from recml_b200.ops import dense as dense_ops
+from recml_b200.ops import mamba_mix
 from recml_b200.ops import norm as norm_ops
 from recml_b200.ops import ssd as ssd_ops
 
@@ -64,8 +65,14 @@ class Mamba2(layer_utils.Configurable, nn.Module):
     a = -torch.exp(self.a_log.float())
     z = dense_ops.linear(inputs, self.z_proj, self.z_bias)
     xbc = dense_ops.linear(inputs, self.xbc_proj, self.xbc_bias)
-    dt = torch.nn.functional.softplus(dense_ops.linear(inputs, self.dt_proj, self.dt_proj_bias).float() + self.dt_bias)
+    dt = dense_ops.linear(inputs, self.dt_proj, self.dt_proj_bias)
     xbc = ssd_ops.conv1d_silu(xbc, self.conv_weight, self.conv_bias)
+    if self.init_states is None and inputs.dtype == torch.bfloat16 and mamba_mix.supported(xbc, z, self.nheads, self.headdim,
+                                                                                          self.d_state):
+      y = mamba_mix.ssd_mix(xbc, dt, self.dt_bias, a, self.headdim)
+      y = mamba_mix.gated_rms_norm(y, z, self.norm_w, self.norm_b, 1e-5)
+      return dense_ops.linear(y, self.out_proj, self.out_bias)
+    dt = torch.nn.functional.softplus(dt.float() + self.dt_bias)
     x, b, c = torch.split(xbc.float(), [self.d_inner, self.d_state, self.d_state], dim=-1)
     x = x.reshape(B, L, self.nheads, self.headdim)
     b = b.reshape(B, L, 1, self.d_state)

@@ -22,7 +22,7 @@ class NativeError(RuntimeError):
 # Number of this library's kernels launched so far (benchmarks reset and read it).  Each launcher
 # call counts the kernels it launches (the radix sort: four per pass, counted by its caller).
 LAUNCHES = {"count": 0}
-_KERNELS_PER_CALL = {"recml_emb_bwd_update": 2, "recml_pack_index": 2, "recml_pair_bce_fwd": 2, "recml_allreduce_bucket": 3, "recml_radix_sort_scratch_words": 0,
+_KERNELS_PER_CALL = {"recml_emb_bwd_update": 2, "recml_pack_index": 2, "recml_mamba_pre_fwd": 2, "recml_mamba_pre_bwd": 2, "recml_pair_bce_fwd": 2, "recml_allreduce_bucket": 3, "recml_radix_sort_scratch_words": 0,
                      "recml_radix_sort_passes": 0, "recml_id_unique_scratch_words": 0, "recml_id_unique_sorted": 3,
                      "recml_emb_bucketize_struct_size": 0,
                      "recml_emb_struct_sizes": 0, "recml_optim_struct_sizes": 0, "recml_ar_struct_sizes": 0,
