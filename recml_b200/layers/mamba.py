@@ -102,9 +102,12 @@ class Mamba2Block(layer_utils.Configurable, nn.Module):
   def forward(self, inputs, padding_mask=None):
     x = self.mamba_dropout(self.mamba_ssm(inputs)).to(inputs.dtype)
     x = norm_ops.layer_norm(x + inputs, self.ln_w, self.ln_b, 1e-12)
-    h = self.drop1(torch.nn.functional.gelu(dense_ops.linear(x, self.ffn_in, self.ffn_in_bias)))
-    y = self.drop2(dense_ops.linear(h, self.ffn_out, self.ffn_out_bias)).to(x.dtype)
-    y = norm_ops.layer_norm(y + x, self.final_ln_w, self.final_ln_b, self.norm_eps)
+    if self.training and (self.drop1.p > 0 or self.drop2.p > 0):
+      h = self.drop1(torch.nn.functional.gelu(dense_ops.linear(x, self.ffn_in, self.ffn_in_bias)))
+      y = self.drop2(dense_ops.linear(h, self.ffn_out, self.ffn_out_bias)).to(x.dtype) + x
+    else:
+      y = dense_ops.gelu_ffn(x, self.ffn_in, self.ffn_in_bias, self.ffn_out, self.ffn_out_bias, erf=True).to(x.dtype) + x
+    y = norm_ops.layer_norm(y, self.final_ln_w, self.final_ln_b, self.norm_eps)
     if padding_mask is not None:
       y = torch.where(padding_mask.bool()[..., None], y, torch.zeros_like(y))
     return y

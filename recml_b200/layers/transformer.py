@@ -34,8 +34,8 @@ class MultiHeadAttention(nn.Module):
     self.out_bias = nn.Parameter(torch.zeros(model_dim))
 
   def forward(self, x: torch.Tensor, mask: torch.Tensor | None, *, padding_mask: torch.Tensor | None = None,
-              causal: bool = False, structured: bool = False) -> torch.Tensor:
-    """`structured` says that `mask` is exactly padding ∧ causality (no explicit attention mask), which
+              causal: bool = False, structured: bool = False, residual: torch.Tensor | None = None) -> torch.Tensor:
+    """`residual` is added to the output projection.  `structured` says that `mask` is exactly padding ∧ causality (no explicit attention mask), which
     lets the op use the packed-sequence kernels instead of a dense `[B, L, L]` mask."""
     B, L, D = x.shape
     qkv = dense_ops.linear(x, self.qkv, self.qkv_bias).reshape(B, L, 3, self.num_heads, self.head_dim)
@@ -44,7 +44,7 @@ class MultiHeadAttention(nn.Module):
     else:
       q, k, v = qkv.unbind(dim=2)
       a = sm_ops.softmax_attention(q, k, v, mask, self.dropout_p, self.training)
-    return dense_ops.linear(a.reshape(B, L, D), self.out, self.out_bias)
+    return dense_ops.linear(a.reshape(B, L, D), self.out, self.out_bias, residual=residual)
 
 
 class TransformerBlock(nn.Module):
@@ -72,11 +72,28 @@ class TransformerBlock(nn.Module):
     ln = norm_ops.layer_norm
     kw = dict(padding_mask=padding_mask, causal=self.causal, structured=attention_mask is None)
     if self.normalize_first:
-      x = x + self.attn_dropout(self.attn(ln(x, self.attn_norm_w, self.attn_norm_b, self.eps), mask, **kw)).to(x.dtype)
-      h = self.activation(dense_ops.linear(ln(x, self.ffn_norm_w, self.ffn_norm_b, self.eps), self.ffn_in,
-                                           self.ffn_in_bias))
-      return x + self.ffn_dropout(dense_ops.linear(h, self.ffn_out, self.ffn_out_bias)).to(x.dtype)
-    x = ln(x + self.attn_dropout(self.attn(x, mask, **kw)).to(x.dtype), self.attn_norm_w, self.attn_norm_b, self.eps)
-    h = self.activation(dense_ops.linear(x, self.ffn_in, self.ffn_in_bias))
-    return ln(x + self.ffn_dropout(dense_ops.linear(h, self.ffn_out, self.ffn_out_bias)).to(x.dtype),
-              self.ffn_norm_w, self.ffn_norm_b, self.eps)
+      x = self._attend(x, ln(x, self.attn_norm_w, self.attn_norm_b, self.eps), mask, kw)
+      return self._feed_forward(x, ln(x, self.ffn_norm_w, self.ffn_norm_b, self.eps))
+    x = ln(self._attend(x, x, mask, kw), self.attn_norm_w, self.attn_norm_b, self.eps)
+    return ln(self._feed_forward(x, x), self.ffn_norm_w, self.ffn_norm_b, self.eps)
+
+  @staticmethod
+  def _fuse_residual(x, dropout: nn.Dropout) -> bool:
+    """A bf16 residual can be added in the epilogue of the product before it when no dropout stands between."""
+    return x.is_cuda and x.dtype == torch.bfloat16 and not (dropout.training and dropout.p > 0)
+
+  def _attend(self, x, inner, mask, kw):
+    """x + dropout(attention(inner))."""
+    if self._fuse_residual(x, self.attn_dropout):
+      return self.attn(inner, mask, residual=x, **kw).to(x.dtype)
+    return x + self.attn_dropout(self.attn(inner, mask, **kw)).to(x.dtype)
+
+  def _feed_forward(self, x, inner):
+    """x + dropout(FFN(inner))."""
+    res = x if self._fuse_residual(x, self.ffn_dropout) else None
+    if self.activation is utils.gelu_approximate:
+      y = dense_ops.gelu_ffn(inner, self.ffn_in, self.ffn_in_bias, self.ffn_out, self.ffn_out_bias, residual=res)
+    else:
+      h = self.activation(dense_ops.linear(inner, self.ffn_in, self.ffn_in_bias))
+      y = dense_ops.linear(h, self.ffn_out, self.ffn_out_bias, residual=res)
+    return y.to(x.dtype) if res is not None else x + self.ffn_dropout(y).to(x.dtype)

@@ -330,9 +330,7 @@ class LinearFn(torch.autograd.Function):
       x2 = x2.to(torch.bfloat16).contiguous()
     w16 = bf16_weight(w)
     if residual is not None:
-      r2 = residual.detach().reshape(-1, w.shape[0])
-      if r2.dtype != torch.bfloat16 or r2.stride(-1) != 1 or r2.stride(0) % 8:
-        r2 = r2.to(torch.bfloat16).contiguous()
+      r2 = _bf16_rows(residual.detach().reshape(-1, w.shape[0]))
       y = G.gemm(x2, w16, bias=None if b is None else b.detach(), epi=G.EPI_ADD, aux0=r2)
     else:
       y = G.gemm(x2, w16, bias=None if b is None else b.detach(), relu=relu)
@@ -365,3 +363,56 @@ def linear(x: torch.Tensor, w: torch.Tensor, b: torch.Tensor | None = None, relu
     return y if residual is None else y + residual.to(y.dtype)
   assert not (relu and residual is not None)
   return LinearFn.apply(x, w, b, relu, residual)
+
+
+def _bf16_rows(x: torch.Tensor) -> torch.Tensor:
+  """`x [M, K]` as bf16 rows on 16-byte boundaries (itself where it is that)."""
+  x = x.to(torch.bfloat16)
+  ok = x.stride(-1) == 1 and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0
+  return x if ok else x.clone(memory_format=torch.contiguous_format)
+
+
+class GeluFfnFn(torch.autograd.Function):
+  """y = gelu(x W1^T + b1) W2^T + b2 (+ residual) with one pass for the activation and one for its derivative.  (Both in
+  the products' epilogues measured slower: a larger epilogue slows every product of that kernel.)"""
+
+  @staticmethod
+  def forward(ctx, x, w1, b1, w2, b2, erf, residual):
+    shp = x.shape
+    x2 = _bf16_rows(x.detach().reshape(-1, shp[-1]))
+    w1_16, w2_16 = bf16_weight(w1), bf16_weight(w2)
+    det = lambda t: None if t is None else t.detach()
+    z = G.gemm(x2, w1_16, bias=det(b1))
+    h = ew.gelu(z, erf)
+    if residual is None:
+      y = G.gemm(h, w2_16, bias=det(b2))
+    else:
+      y = G.gemm(h, w2_16, bias=det(b2), epi=G.EPI_ADD, aux0=_bf16_rows(residual.detach().reshape(-1, w2.shape[0])))
+    ctx.save_for_backward(x2, h, z)
+    ctx.w16 = (w1_16, w2_16)
+    ctx.meta = (shp, x.dtype, w1.dtype, w2.dtype, b1 is not None, b2 is not None, erf,
+                None if residual is None else (residual.shape, residual.dtype))
+    return y.view(*shp[:-1], w2.shape[0])
+
+  @staticmethod
+  def backward(ctx, dy):
+    x2, h, z = ctx.saved_tensors
+    w1_16, w2_16 = ctx.w16
+    shp, xdt, w1dt, w2dt, has_b1, has_b2, erf, res = ctx.meta
+    g = _bf16_rows(dy.reshape(-1, dy.shape[-1]))
+    dw2 = G.gemm(g, h, a_mn=True, b_mn=True, out_dtype=torch.float32)
+    db2 = ew.colsum(g) if has_b2 else None
+    dz = ew.gelu_bwd(G.gemm(g, w2_16, b_mn=True), z, erf)
+    dw1 = G.gemm(dz, x2, a_mn=True, b_mn=True, out_dtype=torch.float32)
+    db1 = ew.colsum(dz) if has_b1 else None
+    dx = G.gemm(dz, w1_16, b_mn=True).view(shp).to(xdt)
+    dres = None if res is None else dy.reshape(res[0]).to(res[1])
+    return dx, dw1.to(w1dt), db1, dw2.to(w2dt), db2, None, dres
+
+
+def gelu_ffn(x: torch.Tensor, w1, b1, w2, b2, erf: bool = False, residual: torch.Tensor | None = None) -> torch.Tensor:
+  """gelu(x w1^T + b1) w2^T + b2 (+ residual): the tanh form of the activation, or the erf form."""
+  if not x.is_cuda or any(n % 8 for n in (*w1.shape, *w2.shape)):
+    h = torch.nn.functional.gelu(linear(x, w1, b1), approximate="none" if erf else "tanh")
+    return linear(h, w2, b2, residual=residual)
+  return GeluFfnFn.apply(x, w1, b1, w2, b2, erf, residual)

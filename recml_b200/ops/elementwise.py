@@ -118,6 +118,23 @@ def silu_bwd_gather4(z, g0, g1_f32, g2, g3):
   return dz
 
 
+def _gelu(z, dy, erf: bool):
+  out = torch.empty_like(z)
+  _lib.check_rc(_lib.cuda().recml_gelu_bf16(_lib.ptr(z), _lib.ptr(dy), _lib.ptr(out), c_ll(z.numel()), c_int(int(erf)),
+                                            _lib.stream()), "gelu")
+  return out
+
+
+def gelu(z: torch.Tensor, erf: bool) -> torch.Tensor:
+  """GELU (erf or tanh form) of a contiguous bf16 CUDA tensor whose element count is a multiple of 8."""
+  return _gelu(z, None, erf)
+
+
+def gelu_bwd(dy: torch.Tensor, z: torch.Tensor, erf: bool) -> torch.Tensor:
+  """dy * gelu'(z), both as `gelu` takes them."""
+  return _gelu(z, dy, erf)
+
+
 def gemv_fwd(x, w, bias):
   """fp32 `[M]` = bf16 `[M, K]` · fp32 `[K]` + bias."""
   if not x.is_cuda:

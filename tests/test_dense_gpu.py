@@ -150,3 +150,43 @@ def test_colsum_matches_fp32_sum(shape, ld):
   # accumulation into an existing vector
   again = ew.colsum(x, out=got.clone())
   torch.testing.assert_close(again, 2 * want, atol=4e-3 * M ** 0.5, rtol=1e-4)
+
+
+@pytest.mark.parametrize("erf", [False, True])
+@pytest.mark.parametrize("n", [8, 4096, 4104, 1 << 20])
+def test_gelu_passes(n, erf):
+  z = torch.cat([torch.linspace(-12, 12, n - 4), torch.tensor([0.0, -0.0, 3e38, -3e38])]).to(torch.bfloat16)
+  dy = torch.randn(n, generator=torch.Generator().manual_seed(n)).to(torch.bfloat16)
+  h, dz = ew.gelu(z.cuda(), erf).cpu().double(), ew.gelu_bwd(dy.cuda(), z.cuda(), erf).cpu().double()
+  x = z.double().requires_grad_()
+  want = torch.nn.functional.gelu(x, approximate="none" if erf else "tanh")
+  slope, = torch.autograd.grad(want[:-2].sum(), x)
+  want = want.detach()
+  # one rounding to bf16; fp32 arithmetic with approximate exponentials: 2^-18 of x (of the slope, at most 1.13)
+  assert bool(((h - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -18 * z.double().abs() * (z.double().abs() < 40))[:-2].all())
+  assert float(h[-2]) == float(z[-2]) and abs(float(h[-1])) == 0.0
+  err = (dz - dy.double() * slope).abs()
+  assert bool((err <= 2.0 ** -8 * (dy.double() * slope).abs() + 2.0 ** -17 * dy.double().abs())[:-2].all())
+
+
+@pytest.mark.parametrize("erf", [False, True])
+@pytest.mark.parametrize("residual", [False, True])
+def test_gelu_ffn_matches_separate_layers(erf, residual):
+  torch.manual_seed(0)
+  x = torch.randn(3, 50, 64, device="cuda").to(torch.bfloat16)
+  w1, b1, w2, b2 = (torch.randn(*s, device="cuda") * 0.2 for s in ((128, 64), (128,), (64, 128), (64,)))
+  g = torch.randn_like(x)
+  got = []
+  for fused in (True, False):
+    xs = x.clone().requires_grad_()
+    ps = [t.clone().requires_grad_() for t in (w1, b1, w2, b2)]
+    if fused:
+      y = dense.gelu_ffn(xs, *ps, erf=erf, residual=xs if residual else None)
+    else:
+      h = torch.nn.functional.gelu(dense.linear(xs, ps[0], ps[1]), approximate="none" if erf else "tanh")
+      y = dense.linear(h, ps[2], ps[3])
+      y = y + xs if residual else y
+    y.backward(g)
+    got.append([y.detach(), xs.grad] + [t.grad for t in ps])
+  for a, b in zip(*got):                            # places of single bf16 roundings differ (2^-8 of a value at most)
+    assert float((a.float() - b.float()).norm() / b.float().norm()) <= 2.0 ** -7
