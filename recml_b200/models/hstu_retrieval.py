@@ -15,6 +15,7 @@ from recml_b200 import embedding as emb
 from recml_b200.layers import hstu as hstu_layers
 from recml_b200.ops import dense as dense_ops
 from recml_b200.ops import norm as norm_ops
+from recml_b200.ops import rows as row_ops
 from recml_b200.ops import sampled_softmax
 
 
@@ -70,7 +71,7 @@ class HSTURetrieval(nn.Module):
     has no next item).  Returns (mean loss, hit@1 among the sampled candidates)."""
     T = input_ids.numel()
     looked = self.items(self.make_lookup_batch(input_ids, target_ids, negative_ids))   # [cap, 3, D]
-    e_in, e_tg, e_ng = looked[:T, 0], looked[:T, 1], looked[:self.num_negatives, 2]
+    e_in, e_tg, e_ng = row_ops.parts(looked, (T, T, self.num_negatives))
     h = self.encoder.encode_jagged(e_in, seq_offsets, timestamps, normalize_input=True)   # [T, D]
     h = self._unit_rows(h).to(e_in.dtype)
     stride = max(T // max(self.num_in_batch, 1), 1)
@@ -78,7 +79,7 @@ class HSTURetrieval(nn.Module):
     cand = torch.cat([e_ng, e_tg[inb_idx]], dim=0)
     cand = self._unit_rows(cand).to(h.dtype)
     cand_ids = torch.cat([negative_ids, target_ids[inb_idx]])
-    pos = (h.float() * self._unit_rows(e_tg).float()).sum(-1)
+    pos = row_ops.row_dot(h, self._unit_rows(e_tg))
     neg = dense_ops.linear(h, cand)                                                       # [T, C] bf16 on CUDA
     loss, hit = sampled_softmax.sampled_softmax_loss(pos, neg, cand_ids, target_ids, target_weights, self.temperature)
     return loss, hit.detach()
