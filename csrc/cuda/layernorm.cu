@@ -160,8 +160,11 @@ __global__ void __launch_bounds__(256) ln_bwd_kernel(const T* __restrict__ dy, c
 
 // bf16 backward with 16-byte accesses for D % 8 == 0, D <= 256 * NCH: lane l owns columns
 // [c * 256 + 8 l, c * 256 + 8 l + 8) of chunk c.  The dw / db partial sums of a block's 8 warps meet in
-// shared memory, so the global atomics are one per column per block.
-template <int NCH>
+// shared memory, so the global atomics are one per column per block.  Bound by memory: the next row's operands are
+// loaded before the current row is reduced, and what would cost registers (weights, the gate's operands where there is
+// no gate) is read again or left out, so that three blocks fit an SM with it (256 columns, no gate).
+// 21 calls of the HSTU step at 65 k tokens: 739 -> 700 us on a B200.
+template <int NCH, bool GATE>
 __global__ void __launch_bounds__(256) ln_bwd_vec_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
                                                          const __nv_bfloat16* __restrict__ gate, const float* __restrict__ w,
                                                          const float* __restrict__ b, const float* __restrict__ stats,
@@ -171,49 +174,69 @@ __global__ void __launch_bounds__(256) ln_bwd_vec_kernel(const __nv_bfloat16* __
   __shared__ float red[8][2][NCH * 256];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const long long warp = (blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x) >> 5;
-  const long long r0 = warp * rows_per_warp;
-  float aw[NCH][8], ab[NCH][8], wv[NCH][8], bv[NCH][8];
-  bool act[NCH];
+  const long long r0 = warp * rows_per_warp, r1 = min(M, r0 + rows_per_warp);
+  float aw[NCH][8], ab[NCH][8];
 #pragma unroll
-  for (int c = 0; c < NCH; ++c) {
-    const int col = c * 256 + lane * 8;
-    act[c] = col < D;
+  for (int c = 0; c < NCH; ++c)
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      aw[c][j] = 0.f; ab[c][j] = 0.f;
-      wv[c][j] = act[c] ? w[col + j] : 0.f;
-      bv[c][j] = (act[c] && b != nullptr) ? b[col + j] : 0.f;
-    }
-  }
+    for (int j = 0; j < 8; ++j) { aw[c][j] = 0.f; ab[c][j] = 0.f; }
   const float inv_d = 1.f / D;
-  for (long long row = r0; row < min(M, r0 + rows_per_warp); ++row) {
-    const float mean = stats[2 * row], rstd = stats[2 * row + 1];
-    float xh[NCH][8], d[NCH][8], d0[NCH][8];
+  uint4 nx[NCH], nd[NCH], ng[NCH];
+  float2 nst = make_float2(0.f, 0.f);
+  auto on = [&](int c) { return c * 256 + lane * 8 < D; };
+  auto fetch = [&](long long row) {
+    nst = __ldg(reinterpret_cast<const float2*>(stats) + row);
+#pragma unroll
+    for (int c = 0; c < NCH; ++c) {
+      if (!on(c)) continue;
+      const long long off = row * D + c * 256 + lane * 8;
+      nx[c] = __ldg(reinterpret_cast<const uint4*>(x + off));
+      nd[c] = __ldg(reinterpret_cast<const uint4*>(dy + off));
+      if (GATE) ng[c] = __ldg(reinterpret_cast<const uint4*>(gate + off));
+    }
+  };
+  auto load8 = [&](const float* p, int c, float (&v)[8]) {
+    const float4 u = __ldg(reinterpret_cast<const float4*>(p + c * 256 + lane * 8));
+    const float4 t = __ldg(reinterpret_cast<const float4*>(p + c * 256 + lane * 8) + 1);
+    v[0] = u.x; v[1] = u.y; v[2] = u.z; v[3] = u.w; v[4] = t.x; v[5] = t.y; v[6] = t.z; v[7] = t.w;
+  };
+  auto unpack8 = [](const uint4& t, float (&v)[8]) {
+    const uint32_t u[4] = {t.x, t.y, t.z, t.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) { v[2 * j] = bf16_lo(u[j]); v[2 * j + 1] = bf16_hi(u[j]); }
+  };
+  auto pack8 = [](const float (&v)[8]) {
+    return make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
+  };
+  if (r0 < r1) fetch(r0);
+  for (long long row = r0; row < r1; ++row) {
+    const float mean = nst.x, rstd = nst.y;
+    float xh[NCH][8], d[NCH][8];          // normalised row; dy * gate
+    uint4 raw_d[NCH];
     float s1 = 0.f, s2 = 0.f;
 #pragma unroll
     for (int c = 0; c < NCH; ++c) {
-      if (!act[c]) continue;
-      const long long off = row * D + c * 256 + lane * 8;
-      const uint4 xv = __ldg(reinterpret_cast<const uint4*>(x + off));
-      const uint4 dv = __ldg(reinterpret_cast<const uint4*>(dy + off));
-      const uint32_t xw[4] = {xv.x, xv.y, xv.z, xv.w}, dwv[4] = {dv.x, dv.y, dv.z, dv.w};
-      uint32_t gw[4] = {0x3f803f80u, 0x3f803f80u, 0x3f803f80u, 0x3f803f80u};   // bf16 ones
-      if (gate != nullptr) {
-        const uint4 gv = __ldg(reinterpret_cast<const uint4*>(gate + off));
-        gw[0] = gv.x; gw[1] = gv.y; gw[2] = gv.z; gw[3] = gv.w;
-      }
+      if (!on(c)) continue;
+      unpack8(nx[c], xh[c]);
+      unpack8(nd[c], d[c]);
+      if (GATE) {
+        float g[8];
+        unpack8(ng[c], g);
+        raw_d[c] = nd[c];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        xh[c][2 * j] = (bf16_lo(xw[j]) - mean) * rstd;
-        xh[c][2 * j + 1] = (bf16_hi(xw[j]) - mean) * rstd;
-        d0[c][2 * j] = bf16_lo(dwv[j]);
-        d0[c][2 * j + 1] = bf16_hi(dwv[j]);
-        d[c][2 * j] = d0[c][2 * j] * bf16_lo(gw[j]);
-        d[c][2 * j + 1] = d0[c][2 * j + 1] * bf16_hi(gw[j]);
+        for (int j = 0; j < 8; ++j) d[c][j] *= g[j];
       }
+    }
+    if (row + 1 < r1) fetch(row + 1);
+#pragma unroll
+    for (int c = 0; c < NCH; ++c) {
+      if (!on(c)) continue;
+      float wv[8];
+      load8(w, c, wv);
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
-        const float dyh = d[c][j] * wv[c][j];
+        xh[c][j] = (xh[c][j] - mean) * rstd;
+        const float dyh = d[c][j] * wv[j];
         s1 += dyh; s2 += dyh * xh[c][j];
       }
     }
@@ -221,22 +244,24 @@ __global__ void __launch_bounds__(256) ln_bwd_vec_kernel(const __nv_bfloat16* __
     if (rms) s1 = 0.f;
 #pragma unroll
     for (int c = 0; c < NCH; ++c) {
-      if (!act[c]) continue;
+      if (!on(c)) continue;
       const long long off = row * D + c * 256 + lane * 8;
-      float o[8];
+      float wv[8], o[8];
+      load8(w, c, wv);
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
-        o[j] = rstd * (d[c][j] * wv[c][j] - s1 - xh[c][j] * s2);
+        o[j] = rstd * (d[c][j] * wv[j] - s1 - xh[c][j] * s2);
         aw[c][j] += d[c][j] * xh[c][j];
         ab[c][j] += d[c][j];
       }
-      *reinterpret_cast<uint4*>(dx + off) =
-          make_uint4(pack_bf16(o[0], o[1]), pack_bf16(o[2], o[3]), pack_bf16(o[4], o[5]), pack_bf16(o[6], o[7]));
-      if (dgate != nullptr) {
+      *reinterpret_cast<uint4*>(dx + off) = pack8(o);
+      if (GATE && dgate != nullptr) {
+        float d0[8], bv[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        unpack8(raw_d[c], d0);
+        if (b != nullptr) load8(b, c, bv);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) o[j] = d0[c][j] * (xh[c][j] * wv[c][j] + bv[c][j]);
-        *reinterpret_cast<uint4*>(dgate + off) =
-            make_uint4(pack_bf16(o[0], o[1]), pack_bf16(o[2], o[3]), pack_bf16(o[4], o[5]), pack_bf16(o[6], o[7]));
+        for (int j = 0; j < 8; ++j) o[j] = d0[j] * (xh[c][j] * wv[j] + bv[j]);
+        *reinterpret_cast<uint4*>(dgate + off) = pack8(o);
       }
     }
   }
@@ -311,20 +336,18 @@ extern "C" int recml_layernorm_bwd(const void* dy, const void* x, const void* ga
   if (M <= 0) return 0;
   if (D > 1024) return -10;
   const bool aligned = ((reinterpret_cast<uintptr_t>(dy) | reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(gate) |
-                         reinterpret_cast<uintptr_t>(dx) | reinterpret_cast<uintptr_t>(dgate)) & 15) == 0;
+                         reinterpret_cast<uintptr_t>(dx) | reinterpret_cast<uintptr_t>(dgate) | reinterpret_cast<uintptr_t>(w) |
+                         reinterpret_cast<uintptr_t>(b) | (reinterpret_cast<uintptr_t>(stats) & 7)) & 15) == 0;
   if (is_bf16 && D % 8 == 0 && D <= 512 && aligned) {
     using B = __nv_bfloat16;
     const int rows_per_warp = M > 148LL * 64 * 4 ? 8 : 2;
     const long long warps = (M + rows_per_warp - 1) / rows_per_warp;
     const int blocks = static_cast<int>((warps + 7) / 8);
-    if (D <= 256)
-      ln_bwd_vec_kernel<1><<<blocks, 256, 0, stream>>>(static_cast<const B*>(dy), static_cast<const B*>(x), static_cast<const B*>(gate),
-                                                       w, b, stats, static_cast<B*>(dx), static_cast<B*>(dgate), dw, db, M, D, rms,
-                                                       rows_per_warp);
-    else
-      ln_bwd_vec_kernel<2><<<blocks, 256, 0, stream>>>(static_cast<const B*>(dy), static_cast<const B*>(x), static_cast<const B*>(gate),
-                                                       w, b, stats, static_cast<B*>(dx), static_cast<B*>(dgate), dw, db, M, D, rms,
-                                                       rows_per_warp);
+#define RECML_LNB(N, G) ln_bwd_vec_kernel<N, G><<<blocks, 256, 0, stream>>>(static_cast<const B*>(dy), static_cast<const B*>(x), \
+      static_cast<const B*>(gate), w, b, stats, static_cast<B*>(dx), static_cast<B*>(dgate), dw, db, M, D, rms, rows_per_warp)
+    if (D <= 256) { if (gate != nullptr) RECML_LNB(1, true); else RECML_LNB(1, false); }
+    else { if (gate != nullptr) RECML_LNB(2, true); else RECML_LNB(2, false); }
+#undef RECML_LNB
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
   }
   if (is_bf16) launch_bwd<__nv_bfloat16>(dy, x, gate, w, b, stats, dx, dgate, dw, db, M, D, rms, stream);
