@@ -507,11 +507,52 @@ static int launch(const void* a, int lda, const void* b, int ldb, const Params& 
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }
 
+// ---- tile width and K split ----------------------------------------------------------------------------------------
+// Tiles of one CTA per SM are handed out in waves, so what counts is how full the last wave is.
+// bf16 results: a 128-wide tile takes about 0.6 of the time of a 256-wide one (it loads A twice as often), so it is
+// taken when that makes fewer or smaller waves: [4224, 512, K 3456] has 66 wide tiles for 148 SMs, 36.9 us, and 132
+// narrow ones, 28.7 us; [8192, 512, K 3456] fits one wave of wide tiles, 41.0 against 47.1 us.  Products whose epilogue
+// streams auxiliary operands through the tile are bound by that epilogue when K is short, and then twice as many
+// half-width tiles keep more of it in flight and balance the last wave.
+static bool wide_tiles(long long M, long long N, long long K, bool aux) {
+  if (N <= 128) return false;
+  const long long sms = sm_count(), mt = (M + BM - 1) / BM;
+  const long long t256 = mt * ((N + 255) / 256), t128 = mt * ((N + 127) / 128);
+  if (aux && K <= 1024 && t256 < 8 * sms) return false;
+  return 3 * ((t128 + sms - 1) / sms) >= 5 * ((t256 + sms - 1) / sms);
+}
+
+// fp32 results without an epilogue (weight gradients: few tiles, very long K) may split K over several CTAs, which add
+// their partial results with atomics to a cleared output.  The model (microseconds) was fitted to sweeps of 9 output
+// shapes x 3 depths x 13 splits x both widths: a k-block takes 0.36 to 0.50 as the wave fills (0.29 to 0.38 for a narrow
+// tile), a wave 3 more, clearing 2, and the atomics pass at 1 TB/s (3 when nothing else runs, but weight gradients run
+// beside the embedding update).  [512, 1024, K 65536]: 16 splits 101 us, the 8 chosen here 83 us.
+static void plan_split(long long M, long long N, long long K, bool* wide, int* split) {
+  static const int tries[] = {1, 2, 3, 4, 5, 6, 8, 10, 12, 16, 24, 32};
+  const long long sms = sm_count(), mt = (M + BM - 1) / BM, kb = (K + BK - 1) / BK;
+  double best = 1e300;
+  *wide = N > 128;
+  *split = 1;
+  for (int w = N > 128 ? 1 : 0; w >= 0; --w) {
+    const long long tiles = mt * (w ? (N + 255) / 256 : (N + 127) / 128);
+    for (int s : tries) {
+      if (s > 1 && kb < 4LL * s) break;
+      const long long waves = (tiles * s + sms - 1) / sms;
+      const double full = static_cast<double>(tiles * s) / (waves * sms);
+      double cost = waves * (((kb + s - 1) / s) * (w ? 0.36 + 0.14 * full : 0.29 + 0.09 * full) + 3.0);
+      if (s > 1) cost += 2.0 + static_cast<double>(s) * M * N * 4.0 / 1.0e6;
+      if (cost < best) { best = cost; *wide = w != 0; *split = s; }
+    }
+  }
+}
+
 }  // namespace gemm
 }  // namespace recml
 
 // D[M,N] = epi(A·B^T).  a_mn / b_mn: 0 = operand stored [rows, K] (K contiguous), 1 = stored [K, rows].
 // Leading dims are in elements and must be multiples of 8 (16-byte TMA strides); N must be a multiple of 8.
+// split_k: 1 or more as given (the caller clears an output that is not accumulated into); 0 lets the plan above choose
+// for an fp32 output without an epilogue, and clears the output here when it is split.
 // Returns 0 on a successful launch, negative on bad arguments / set-up failure.
 extern "C" int recml_gemm_bf16(const void* a, int lda, int a_mn, const void* b, int ldb, int b_mn, void* d,
                                int ldd, int out_f32, int accumulate, int M, int N, int K, const float* bias,
@@ -529,21 +570,22 @@ extern "C" int recml_gemm_bf16(const void* a, int lda, int a_mn, const void* b, 
   p.bias = bias; p.relu = relu; p.epi = epi;
   p.aux0 = static_cast<const __nv_bfloat16*>(aux0); p.aux1 = static_cast<const __nv_bfloat16*>(aux1);
   p.ldaux = ldaux; p.out2 = static_cast<__nv_bfloat16*>(out2); p.status = status;
+  const bool plain_f32 = out_f32 && epi == kEpiLinear && bias == nullptr && !relu;
+  bool wide = wide_tiles(M, N, K, epi != kEpiLinear);
+  static const int forced_bn = [] { const char* e = getenv("RECML_GEMM_BN"); return e ? atoi(e) : 0; }();
+  const bool planned = split_k == 0 && plain_f32;
+  if (planned) plan_split(M, N, K, &wide, &split_k);
   {
     const int kb = (K + BK - 1) / BK;
     if (split_k > kb) split_k = kb;
-    if (split_k > 1 && (!out_f32 || epi != kEpiLinear || bias != nullptr || relu)) return -13;
+    if (split_k > 1 && !plain_f32) return -13;
     // every split must own at least one k-block
     while (split_k > 1 && ((kb + split_k - 1) / split_k) * (split_k - 1) >= kb) --split_k;
     p.split_k = split_k > 1 ? split_k : 1;
   }
-  // Tile width: 256 columns amortise the operand traffic of long-K products; products whose epilogue streams
-  // auxiliary operands through the tile (cross / add / mask epilogues) are bound by that epilogue when K is
-  // short, and then twice as many half-width tiles keep more of it in flight and balance the last wave.
-  static const int forced_bn = [] { const char* e = getenv("RECML_GEMM_BN"); return e ? atoi(e) : 0; }();
-  bool wide = N > 128;
-  if (wide && epi != kEpiLinear && !out_f32 && K <= 1024 &&
-      static_cast<long long>((M + BM - 1) / BM) * ((N + 255) / 256) < 8LL * sm_count()) wide = false;
+  if (planned && p.split_k > 1 && !accumulate &&
+      cudaMemset2DAsync(d, static_cast<size_t>(ldd) * 4, 0, static_cast<size_t>(N) * 4, M, stream) != cudaSuccess)
+    return -4;
   if (forced_bn == 128) wide = false;
   if (forced_bn == 256) wide = N > 128;
   if (!a_mn && !b_mn) return wide ? launch<256, false, false>(a, lda, b, ldb, p, stream)

@@ -53,7 +53,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
          aux0: torch.Tensor | None = None, aux1: torch.Tensor | None = None,
          out_dtype: torch.dtype = torch.bfloat16, out: torch.Tensor | None = None,
          accumulate_into: torch.Tensor | None = None, want_out2: bool = False, split_k: int = 0):
-  """`split_k=0` picks a K split automatically for fp32-output products whose tile count would
+  """`split_k=0` lets the launcher pick a K split for fp32-output products whose tile count would
   leave most SMs idle (weight gradients: few output tiles, very long K)."""
   if not a.is_cuda:
     return gemm_reference(a, b, a_mn=a_mn, b_mn=b_mn, bias=bias, relu=relu, epi=epi, aux0=aux0,
@@ -71,13 +71,6 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
     d = out if out is not None else _lib.debug_empty((M, N), out_dtype, a.device, f"gemm output [{M}, {N}]")
     out_f32, acc = int(d.dtype == torch.float32), 0
   out2 = _lib.debug_empty((M, N), torch.bfloat16, a.device, "gemm second output") if want_out2 else None
-  if split_k == 0:
-    split_k = 1
-    if out_f32 and epi == EPI_LINEAR and bias is None and not relu:
-      tiles = ((M + 127) // 128) * ((N + 255) // 256 if N > 128 else 1)
-      kb = (K + 63) // 64
-      if tiles < 148 and kb >= 32:
-        split_k = max(1, min(296 // tiles, kb // 16, 16))
   if split_k > 1 and not acc:
     d.zero_()
   ldaux = aux0.stride(0) if aux0 is not None else 0

@@ -87,3 +87,39 @@ def test_checked_build_guard_words():
                        cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
   assert out.returncode == 0, out.stderr[-2000:]
   assert "CAUGHT" in out.stdout and "probe" in out.stdout
+
+
+@pytest.mark.parametrize("M,N,K", [(128, 128, 4096), (136, 264, 8192), (512, 16, 4224), (256, 512, 4224), (1024, 1024, 2112),
+                                   (3456, 512, 512), (8, 8, 8), (64, 136, 255 * 8)])
+@pytest.mark.parametrize("accumulate", [False, True])
+def test_planned_split_into_a_wider_output(M, N, K, accumulate):
+  """The launcher's own choice of tile width and K split, into columns of a wider matrix: what lies beside them stays."""
+  g = torch.Generator().manual_seed(M + N + K)
+  a, b = (torch.randn(K, n, generator=g).to(torch.bfloat16) for n in (M, N))
+  full = torch.randn(M, N + 24, generator=g)
+  out = full.cuda()
+  view = out[:, 8:8 + N]
+  if accumulate:
+    G.gemm(a.cuda(), b.cuda(), a_mn=True, b_mn=True, accumulate_into=view)
+  else:
+    G.gemm(a.cuda(), b.cuda(), a_mn=True, b_mn=True, out=view)
+  torch.cuda.synchronize()
+  _lib.check_status()
+  want = full.double()
+  want[:, 8:8 + N] = a.double().t() @ b.double() + (want[:, 8:8 + N] if accumulate else 0.0)
+  # fp32 sums of K exact products: K roundings of the sum of magnitudes at most
+  bound = torch.zeros_like(want)
+  bound[:, 8:8 + N] = (K + 4) * 2.0 ** -24 * (a.double().abs().t() @ b.double().abs() + full[:, 8:8 + N].double().abs())
+  assert bool(((out.cpu().double() - want).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("M,N,K", [(4224, 512, 136), (8192, 256, 64), (300, 512, 3456), (18944, 256, 64), (19000, 264, 72)])
+@pytest.mark.parametrize("epi", [G.EPI_LINEAR, G.EPI_ADD, G.EPI_CROSS])
+def test_tile_width_choices(M, N, K, epi):
+  """Shapes on both sides of the tile-width rule (one wave of narrow tiles, full waves of wide ones, ragged edges)."""
+  a, b, x0, x1 = _rand(M, K), _rand(N, K), _rand(M, N), _rand(M, N)
+  kw = {} if epi == G.EPI_LINEAR else dict(epi=epi, aux0=x0, aux1=x1)
+  out = G.gemm(a, b, want_out2=epi == G.EPI_CROSS, **kw)
+  ref = G.gemm_reference(a, b, want_out2=epi == G.EPI_CROSS, out_dtype=torch.float32, **kw)
+  for o, r in zip(*((out, ref) if epi == G.EPI_CROSS else ((out,), (ref,)))):
+    _check(o, r)
