@@ -444,7 +444,8 @@ struct FwdParams {
                             // counted here (allow_id_dropping); null: an overflow is a kCapacity error
   int prefetch;             // bit 0: ask L2 for a bag's rows as soon as their ids are known; bit 1 (tiled kernel):
                             // let owned ids wait in the warp's queue across chunks
-  int tiled;                // 1: no sequence feature in this launch -> the bags-in-tiles kernel
+  int tiled;                // 1: no sequence feature in this launch -> a bags-in-tiles kernel; 2: and the destination
+                            //    columns of every feature start on 8-byte boundaries
   long long total_tiles;    // tiled: sum over features of W * ceil(B / bags per tile)
   int prefiltered;          // 1: the senders bucketized the ids: every id of a row-sharded pooled feature found here
                             //    is owned (sequence features keep their positions, so they still arrive whole)
@@ -799,6 +800,171 @@ __global__ void __launch_bounds__(256, 2) emb_fwd_tiled_kernel(const FwdParams p
     store_upto(nb);       // the open bag and the (empty or un-owned) bags after it
   }
   grid_done_then_signal(p.done_counter, p.flags, p.W, seq);
+}
+
+// ---- forward, tiled, one rank: several walkers per warp ------------------------------------------------
+// On one rank every valid id is owned, so nothing has to be sorted out or queued.  G lanes of eight columns take a row
+// (16 lanes for 128 columns) and a warp's 32 / G walkers share the bags of a tile: the kernel above is bound by the
+// instructions around each row (105 to 150 ps per row whatever its width), and these now serve 32 / G rows.  Control
+// flow is uniform over the warp.  The tile's occurrence entries are claimed together, after a pass that counts.
+// On a B200: DLRM step of 65536 samples 11.93 -> 11.30 ms, of 8192 samples 1.957 -> 1.878 ms, of 4224 samples
+// 1.280 -> 1.224 ms; jagged mean-pooled lookup and update of 1.57 M ids x 64 columns 583 -> 464 us.
+template <int G, bool TRAIN, bool GAINS>
+__global__ void __launch_bounds__(256, 3) emb_fwd_walk_kernel(const FwdParams p) {
+  constexpr unsigned int kAll = 0xffffffffu;
+  constexpr int kWalkers = 32 / G;
+  constexpr int kBatch = 4;
+  const int lane = threadIdx.x & 31, sub = lane % G, grp = lane / G;
+  const unsigned int group_bits = G == 32 ? kAll : (1u << (G & 31)) - 1u;
+  const long long warps = (static_cast<long long>(gridDim.x) * blockDim.x) >> 5;
+  const bool lane_on = sub * 8 < p.dloc;
+  const int* vals = p.ids.values[0];
+  const float* wts = GAINS ? p.ids.weights[0] : nullptr;
+  for (long long tile = (blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x) >> 5; tile < p.total_tiles; tile += warps) {
+    int fi = -1;
+    for (int f0 = 0; f0 < p.n_feats; f0 += 32) {
+      const int fx = f0 + lane;
+      fi += __popc(__ballot_sync(kAll, fx < p.n_feats && p.feats[fx].tile_start <= tile));
+    }
+    const FeatDesc& f = p.feats[fi];
+    const int bpt = 1 << f.tile_shift, row_base = f.row_base, vocab = f.vocab, combiner = f.combiner;
+    const long long dst_stride = f.dst_stride, grad_off = f.grad_off;
+    const int tile0 = static_cast<int>(tile - f.tile_start) << f.tile_shift;
+    const int tile_nb = min(bpt, p.B - tile0);                   // bags of the tile, shared out among the walkers
+    const int per = (tile_nb + kWalkers - 1) / kWalkers;         // <= G
+    const int b0 = tile0 + min(grp * per, tile_nb);
+    const int nb = max(0, min(per, tile_nb - grp * per));
+    const int* offs = p.ids.offsets[0] + static_cast<long long>(f.feat_index) * p.B + b0;
+    const int o_mine = offs[min(sub, nb)];                       // first id of bag `sub` (lanes >= nb: the end)
+    const int p0 = __shfl_sync(kAll, o_mine, 0, G);
+    const int p1 = offs[nb];
+    float scale_mine = 1.f;
+    if (GAINS && combiner != kSum) {                             // combiner denominator of this lane's bag
+      const int o1 = __shfl_down_sync(kAll, o_mine, 1, G);
+      const int e = sub == G - 1 ? p1 : o1;
+      float den = 0.f;
+      if (sub < nb) {
+        for (int i = o_mine; i < e; ++i) {
+          const float w = wts != nullptr ? wts[i] : 1.f;
+          den += combiner == kMean ? w : w * w;
+        }
+      }
+      if (combiner == kSqrtN) den = sqrtf(den);
+      scale_mine = den != 0.f ? 1.f / den : 0.f;
+    }
+    unsigned int pos = 0;                                        // next occurrence entry of this walker
+    if (TRAIN) {
+      unsigned int mine = 0;
+      for (int i = p0 + sub; i < p1; i += G) { const int id = vals[i]; mine += id >= 0 && id < vocab; }
+      // claims in lane order, so that a walker's entries are contiguous
+      unsigned int incl = mine;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const unsigned int v = __shfl_up_sync(kAll, incl, o);
+        if (lane >= o) incl += v;
+      }
+      const unsigned int total = __shfl_sync(kAll, incl, 31);
+      unsigned int first = 0;
+      if (lane == 0 && total != 0) first = atomicAdd(p.occ_count, total);
+      first = __shfl_sync(kAll, first, 0);
+      pos = first + __shfl_sync(kAll, incl - mine, 0, G);        // entries of the walkers before
+    }
+    __nv_bfloat16* dst = p.pooled.p[0] + f.slot_off + (f.kind == kColumnWise ? f.col_lo : 0) + sub * 8 + b0 * dst_stride;
+    Vec<8> acc;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) acc.v[e] = 0.f;
+    int cur = 0;          // bag whose sum is being built; bags below it have been stored
+    auto store_upto = [&](int bag) {      // stores bag `cur` and zeros for the empty ones up to `bag`
+      while (__any_sync(kAll, cur < bag)) {
+        if (cur < bag) {
+          if (lane_on) {
+            uint2* d = reinterpret_cast<uint2*>(dst + cur * dst_stride);
+            d[0] = make_uint2(pack_bf16(acc.v[0], acc.v[1]), pack_bf16(acc.v[2], acc.v[3]));
+            d[1] = make_uint2(pack_bf16(acc.v[4], acc.v[5]), pack_bf16(acc.v[6], acc.v[7]));
+          }
+#pragma unroll
+          for (int e = 0; e < 8; ++e) acc.v[e] = 0.f;
+          ++cur;
+        }
+      }
+    };
+    for (int base = p0; __any_sync(kAll, base < p1); base += G) {
+      const int i = base + sub;
+      const int cnt = max(0, min(G, p1 - base));
+      const int id = i < p1 ? vals[i] : -1;
+      if (id >= vocab) report(p.status, kBadIndex, id);
+      bool owned = id >= 0 && id < vocab;
+      const unsigned int lrow = static_cast<unsigned int>(row_base + id);
+      if (owned && (p.prefetch & 1)) prefetch_l2(p.table + static_cast<size_t>(lrow) * p.dloc, p.dloc * 4);
+      int lo = 0, hi = nb;                                       // o[lo] <= i < o[hi]
+#pragma unroll
+      for (int step = 1; step < G; step <<= 1) {
+        const int mid = (lo + hi) >> 1;
+        const int om = __shfl_sync(kAll, o_mine, mid, G);
+        if (hi - lo > 1) { if (om <= i) lo = mid; else hi = mid; }
+      }
+      const int bag = lo;
+      float w = 1.f;
+      if (GAINS) {
+        const float sc = __shfl_sync(kAll, scale_mine, bag, G);
+        if (i < p1) w = (wts != nullptr ? wts[i] : 1.f) * sc;
+      }
+      if (TRAIN) {
+        const unsigned int m = (__ballot_sync(kAll, owned) >> (lane - sub)) & group_bits;
+        const unsigned int at = pos + __popc(m & ((1u << sub) - 1u));
+        pos += __popc(m);
+        const bool fits = owned && at < p.occ_cap;
+        if (fits) {
+          const long long gvl = p.grad_ld > 0 ? (static_cast<long long>(b0 + bag) * p.grad_ld + grad_off) / 8
+                                              : grad_off / p.dloc + (b0 + bag);
+          const unsigned int gv = static_cast<unsigned int>(gvl);
+          p.occ_key[at] = lrow;
+          if (GAINS) {
+            p.occ_val[at] = at;
+            p.occ_gain[2 * static_cast<size_t>(at)] = __uint_as_float(gv);
+            p.occ_gain[2 * static_cast<size_t>(at) + 1] = w;
+          } else {
+            p.occ_val[at] = gv;
+          }
+        }
+        const unsigned int over = __ballot_sync(kAll, owned && !fits);
+        if (over != 0) {
+          if (p.dropped != nullptr) {
+            if (lane == 0) atomicAdd(p.dropped, static_cast<unsigned int>(__popc(over)));
+            owned = fits;
+          } else if (lane == 0) {
+            report(p.status, kCapacity, 1);
+          }
+        }
+      }
+      const unsigned int row = owned ? lrow : 0xffffffffu;
+      const int cnt_max = __reduce_max_sync(kAll, cnt);
+      for (int j0 = 0; j0 < cnt_max; j0 += kBatch) {
+        Vec<8> r[kBatch];
+#pragma unroll
+        for (int u = 0; u < kBatch; ++u) {
+          const unsigned int rj = __shfl_sync(kAll, row, j0 + u, G);
+#pragma unroll
+          for (int e = 0; e < 8; ++e) r[u].v[e] = 0.f;
+          if (lane_on && rj != 0xffffffffu) r[u] = load_f32<8>(p.table + static_cast<size_t>(rj) * p.dloc + sub * 8);
+        }
+#pragma unroll
+        for (int u = 0; u < kBatch; ++u) {
+          const int j = j0 + u;
+          const unsigned int rj = __shfl_sync(kAll, row, j, G);
+          const int bag_j = __shfl_sync(kAll, bag, j, G), bj = rj != 0xffffffffu ? bag_j : cur;
+          const float wj = GAINS ? __shfl_sync(kAll, w, j, G) : 1.f;
+          if (__any_sync(kAll, bj != cur)) store_upto(bj);
+          if (rj != 0xffffffffu) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) acc.v[e] = GAINS ? fmaf(wj, r[u].v[e], acc.v[e]) : acc.v[e] + r[u].v[e];
+          }
+        }
+      }
+    }
+    store_upto(nb);       // the open bag and the empty ones after it
+  }
+  grid_done_then_signal(p.done_counter, p.flags, p.W, seq_of(p.seq));
 }
 
 // =================================== combine: sum source slots, write concat =======================
@@ -1400,6 +1566,16 @@ extern "C" int recml_emb_push_ids(const PushIdsParams* p, cudaStream_t stream) {
 
 template <int VPL>
 static void launch_fwd(const FwdParams& p, bool train, bool gains, int blocks, cudaStream_t stream) {
+  if (p.tiled == 2 && p.W == 1 && p.wait_flags == nullptr && p.dloc % 8 == 0 && (reinterpret_cast<uintptr_t>(p.table) & 15) == 0) {
+    if (train) {
+      if (gains) emb_fwd_walk_kernel<4 * VPL, true, true><<<blocks, 256, 0, stream>>>(p);
+      else emb_fwd_walk_kernel<4 * VPL, true, false><<<blocks, 256, 0, stream>>>(p);
+    } else {
+      if (gains) emb_fwd_walk_kernel<4 * VPL, false, true><<<blocks, 256, 0, stream>>>(p);
+      else emb_fwd_walk_kernel<4 * VPL, false, false><<<blocks, 256, 0, stream>>>(p);
+    }
+    return;
+  }
   if (p.tiled) {
     if (train) {
       if (gains) emb_fwd_tiled_kernel<VPL, true, true><<<blocks, 256, 0, stream>>>(p);

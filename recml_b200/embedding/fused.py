@@ -403,6 +403,7 @@ class FusedBackend:
       m = self.m
       feats = []
       tiles = 0
+      even = m.world == 1      # destination columns on 8-byte boundaries (see FwdParams.tiled)
       for fname, col, width, L in self.layout:
         if fname not in info["feat_names"]:
           continue
@@ -413,6 +414,7 @@ class FusedBackend:
           slot, goff, stride = out_col + col, out_col + col, ld
         else:
           slot, goff, stride = self.slot_off[fname], self.grad_off[m.rank][fname], width
+        even = even and slot % 4 == 0 and stride % 4 == 0 and tp.col_lo % 4 == 0
         # bags per warp of the tiled forward: a few hundred ids per tile whatever the bag size
         # (of a row-sharded feature a rank receives 1 / W of every bag when the senders bucketize the ids;
         # otherwise it scans all of them and gathers 1 / W: weigh the two)
@@ -428,6 +430,7 @@ class FusedBackend:
         tiles += m.world * ((self.B + bpt - 1) // bpt)
       info["descs"][direct] = _device_struct_array(feats, m.device)
       info["tiles"] = tiles
+      info.setdefault("even", {})[direct] = even
     return info["descs"][direct]
 
   def _ensure_occ(self, kjt):
@@ -457,7 +460,7 @@ class FusedBackend:
                            count=torch.zeros(1, dtype=torch.int32, device=dev), sorted=0)
                       for _ in range(self.pipeline_depth)]
       dloc = m.plan.stacks[si].dim
-      info["range_len"] = update_range(cap, max(1, 256 // dloc) if m.plan.stacks[si].optimizer.kind == "rowwise_adagrad" else 1)
+      info["range_len"] = update_range(cap, max(1, min(8, 256 // dloc)) if m.plan.stacks[si].optimizer.kind == "rowwise_adagrad" else 1)
       info["scratch"] = torch.zeros(-(-cap // info["range_len"]), dloc, dtype=torch.float32, device=dev)
       words = int(self.lib.recml_radix_sort_scratch_words(c_ll(cap)))
       info["sort_scratch"] = torch.empty(words, dtype=torch.int32, device=dev)
@@ -575,6 +578,8 @@ class FusedBackend:
       fp.wait_flags = self._flag_ptr(m.rank, 0, 0) if W > 1 else None
       fp.prefetch = self.fwd_prefetch
       fp.tiled = int(self.fwd_tiled and all(L == 0 for f_, _, _, L in self.layout if f_ in info["feat_names"]))
+      if fp.tiled and info["even"][direct] and fp.pooled[0] % 8 == 0:
+        fp.tiled = 2
       fp.total_tiles = info.get("tiles", 0)
       fp.prefiltered = int(bucket is not None)
       fp.done_counter, fp.seq, fp.status = info["done"].data_ptr(), seq, self.status.data_ptr()

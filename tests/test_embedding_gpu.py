@@ -204,3 +204,28 @@ def test_update_ranges(range_len, opt, dim):
     sum_err = cnt * 2.0 ** -24 * mags.amax(-1, keepdim=True)
     bound = 0.05 * 2 * sum_err / 0.1 ** 0.5 + 8 * 2.0 ** -24 * (table.double().abs() + 1.0)
     assert bool(((t.cpu().double() - want).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("D", [8, 24, 64, 128, 200, 256])
+@pytest.mark.parametrize("B", [1, 31, 33, 130])
+@pytest.mark.parametrize("combiner", ["sum", "mean"])
+def test_lookup_tiles(D, B, combiner):
+  """Bags from none to many windows of ids, tiles that do not fill, features of two widths side by side, and the update
+  of what was looked up."""
+  rng = np.random.default_rng(B + D)
+  vocabs, bags = [40, 900, 300], [1, 12, 90]
+  specs = {f"f{i}": emb.EmbeddingSpec(v, D, combiner=combiner) for i, v in enumerate(vocabs)}
+  if B == 33:
+    specs = {"f0": emb.EmbeddingSpec(vocabs[0], 40, combiner=combiner), **{k: specs[k] for k in ("f1", "f2")}}
+  g, c = _pair(specs, emb.RowWiseAdagradOptimizerSpec(0.05))
+  kjt = _batch(rng, B, vocabs, bags, ragged=True)
+  og, oc = g(kjt.to_device(torch.device("cuda")), flat=True), c(kjt, flat=True)
+  # fp32 sums, one rounding to bf16
+  torch.testing.assert_close(og.float().cpu(), oc.float(), atol=1e-4, rtol=2.0 ** -7)
+  grad = (torch.randn(oc.shape) * 0.1).to(torch.bfloat16).float()
+  oc.backward(grad)
+  og.backward(grad.cuda().to(og.dtype))
+  torch.cuda.synchronize()
+  _lib.check_status()
+  for name in g.plan.tables:
+    torch.testing.assert_close(g.gather_table(name).cpu(), c.gather_table(name), atol=3e-3, rtol=3e-3)
