@@ -397,6 +397,7 @@ __global__ void gemv_bwd_kernel(const __nv_bfloat16* __restrict__ x, long long l
   for (int k = threadIdx.x * 2; k < K; k += 2 * blockDim.x) {
     const float w0 = w[k], w1 = w[k + 1];
     float a0 = 0.f, a1 = 0.f;
+#pragma unroll 4
     for (long long r = r0; r < r1; ++r) {
       const float d = dy[r];
       const uint32_t t = *reinterpret_cast<const uint32_t*>(x + r * ld + k);
@@ -456,8 +457,11 @@ extern "C" int recml_cast_pad_rows(const float* in, int cols_in, void* out, int 
 extern "C" int recml_colsum_bf16(const void* x, long long M, int N, long long ld, float* out, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return 0;
   if (N % 8 == 0 && ld % 8 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0) {
-    const int rows_per_block = 256;
-    dim3 grid((N + 255) / 256, static_cast<unsigned>((M + rows_per_block - 1) / rows_per_block));
+    // about four blocks per SM, with 32 to 256 rows each: [8192, 256] has 256 blocks instead of 32
+    const int cb = (N + 255) / 256;
+    long long rows = (M * cb / (148 * 4) + 31) / 32 * 32;
+    const int rows_per_block = static_cast<int>(rows < 32 ? 32 : rows > 256 ? 256 : rows);
+    dim3 grid(cb, static_cast<unsigned>((M + rows_per_block - 1) / rows_per_block));
     colsum8_kernel<<<grid, 256, 0, stream>>>(static_cast<const __nv_bfloat16*>(x), M, N, ld, out, rows_per_block);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
   }
@@ -551,7 +555,8 @@ extern "C" int recml_gemv_fwd(const void* x, long long ld, int K, const float* w
 extern "C" int recml_gemv_bwd(const void* x, long long ld, int K, const float* w, const float* dy, long long M,
                               void* dx, long long lddx, int mask_relu, float* dw, float* db, cudaStream_t stream) {
   if (M <= 0) return 0;
-  const int rows_per_block = 64;
+  // a block walks its rows one after the other: short walks while that still gives few blocks
+  const int rows_per_block = M <= 148LL * 8 * 16 ? 16 : 64;
   gemv_bwd_kernel<<<static_cast<int>((M + rows_per_block - 1) / rows_per_block), 256, 0, stream>>>(
       static_cast<const __nv_bfloat16*>(x), ld, K, w, dy, M, static_cast<__nv_bfloat16*>(dx), lddx, mask_relu, dw, db,
       rows_per_block);
