@@ -368,7 +368,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, b: torch.Tensor | None = None, relu
 def _bf16_rows(x: torch.Tensor) -> torch.Tensor:
   """`x [M, K]` as bf16 rows on 16-byte boundaries (itself where it is that)."""
   x = x.to(torch.bfloat16)
-  ok = x.stride(-1) == 1 and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0
+  ok = x.stride(-1) == 1 and x.stride(0) % 8 == 0 and x.stride(0) >= x.shape[1] and x.data_ptr() % 16 == 0
   return x if ok else x.clone(memory_format=torch.contiguous_format)
 
 
