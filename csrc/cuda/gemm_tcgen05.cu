@@ -474,6 +474,23 @@ static int make_map(CUtensorMap* map, const void* ptr, int rows, int cols, int l
   return make_map_bf16(map, ptr, rows, cols, ld, box_rows);
 }
 
+// Shared-memory limit of every instance, set at the first product of the process: which instance a shape takes depends
+// on its sizes, and one that is first met later (in a timed step, under stream capture) should be loaded by then.
+static bool configure_all() {
+  const cudaFuncAttribute kMax = cudaFuncAttributeMaxDynamicSharedMemorySize;
+  bool ok = true;
+  auto set = [&](const void* kernel, int bytes) { ok = ok && cudaFuncSetAttribute(kernel, kMax, bytes) == cudaSuccess; };
+  set(reinterpret_cast<const void*>(gemm_kernel<128, false, false>), Cfg<128>::kSmem);
+  set(reinterpret_cast<const void*>(gemm_kernel<128, false, true>), Cfg<128>::kSmem);
+  set(reinterpret_cast<const void*>(gemm_kernel<128, true, false>), Cfg<128>::kSmem);
+  set(reinterpret_cast<const void*>(gemm_kernel<128, true, true>), Cfg<128>::kSmem);
+  set(reinterpret_cast<const void*>(gemm_kernel<256, false, false>), Cfg<256>::kSmem);
+  set(reinterpret_cast<const void*>(gemm_kernel<256, false, true>), Cfg<256>::kSmem);
+  set(reinterpret_cast<const void*>(gemm_kernel<256, true, false>), Cfg<256>::kSmem);
+  set(reinterpret_cast<const void*>(gemm_kernel<256, true, true>), Cfg<256>::kSmem);
+  return ok;
+}
+
 template <int BN, bool A_MN, bool B_MN>
 static int launch(const void* a, int lda, const void* b, int ldb, const Params& p, cudaStream_t stream) {
   CUtensorMap ma, mb;
@@ -495,12 +512,8 @@ static int launch(const void* a, int lda, const void* b, int ldb, const Params& 
   if (!p.out_f32 && p.aux0 != nullptr && make_map(&mx0, p.aux0, p.M, p.N, p.ldaux, 32)) return -5;
   if (!p.out_f32 && p.aux1 != nullptr && make_map(&mx1, p.aux1, p.M, p.N, p.ldaux, 32)) return -5;
   auto kern = gemm_kernel<BN, A_MN, B_MN>;
-  static bool configured = false;
-  if (!configured) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<BN>::kSmem) != cudaSuccess)
-      return -3;
-    configured = true;
-  }
+  static const bool configured = configure_all();
+  if (!configured) return -3;
   const int tiles = ((p.M + BM - 1) / BM) * ((p.N + BN - 1) / BN) * (p.split_k > 1 ? p.split_k : 1);
   const int grid = tiles < sm_count() ? tiles : sm_count();
   kern<<<grid, kThreads, Cfg<BN>::kSmem, stream>>>(ma, mb, md, md2, mx0, mx1, p);
